@@ -1,0 +1,111 @@
+"""The batched FP32 Legendre products (kernels/leg_gemm.cuh) at the sizes where
+their tiles end: 16-degree k-tiles, blocks of 8, 16, 24 and 32 degrees (one or
+two to a parity, one or two CTAs to an order), 64-latitude tiles, 8-, 16- and
+32-field tiles, odd latitudes, mmax < lmax.
+
+Every field is the first one times a power of two, so its result has to be
+the first one's times that power, bit by bit; the first one is checked against
+the f64 oracle (relative L2 <= 1e-5, the plain FP32 path's bound up to lmax 255).
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from turing_sphere_b200 import (GpuModel, ShtConfig, ShtPlan, defaultParams, mModelByKey,
+                                seededNoise)
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+CASES = [
+    (31, 31, 48, 96, 8), (31, 31, 33, 64, 9), (62, 62, 96, 192, 33), (64, 50, 131, 256, 17),
+    (95, 95, 128, 256, 16), (127, 127, 192, 384, 5), (128, 100, 193, 512, 36),
+    (129, 129, 260, 512, 16), (190, 190, 320, 768, 4), (255, 255, 384, 768, 4),
+    (255, 3, 384, 768, 70),
+]
+
+
+def spectrum(lmax, mmax, seed):
+    q = np.random.default_rng(seed).standard_normal((O.nlm_calc(lmax, mmax), 2))
+    l_of = np.concatenate([np.arange(m, lmax + 1) for m in range(mmax + 1)])
+    q /= l_of[:, None] + 1.0
+    q[:lmax + 1, 1] = 0.0  # m = 0
+    return q.astype(np.float32).ravel()
+
+
+@pytest.mark.parametrize("lmax,mmax,nlat,nphi,batch", CASES)
+def test_every_field_of_a_batch(device, parity, lmax, mmax, nlat, nphi, batch):
+    import torch
+    plan = ShtPlan.create(device, ShtConfig(lmax, mmax, nlat, nphi))
+    ref = O.ShtReference(lmax, mmax, nlat, nphi)
+
+    def run(call, x, n):  # one call on device arrays (host arrays go in chunks of fields)
+        src = torch.from_numpy(x).cuda()
+        dst = torch.empty(batch, n, device="cuda")
+        torch.cuda.synchronize()
+        call(src.data_ptr(), dst.data_ptr(), batch)
+        device.sync()
+        return dst.cpu().numpy()
+
+    scale = np.ldexp(np.float32(1), -(np.arange(batch) % 5)).astype(np.float32)[:, None]
+    q = spectrum(lmax, mmax, lmax + batch)
+    grid = run(plan.synth_dev, scale * q[None, :], nlat * nphi)
+    want = ref.synth(q.astype(np.float64))
+    parity(f"leg_gemm synth lmax{lmax} mmax{mmax} nlat{nlat} B{batch}", O.rel_l2(grid[0], want), TOL)
+    assert np.array_equal(grid, scale * grid[0])
+    g = want.astype(np.float32)
+    back = run(plan.analys_dev, scale * g[None, :].reshape(1, -1), q.size)
+    parity(f"leg_gemm analys lmax{lmax} mmax{mmax} nlat{nlat} B{batch}",
+           O.rel_l2(back[0], ref.analys(g.astype(np.float64))), TOL)
+    assert np.array_equal(back, scale * back[0])
+    plan.destroy()
+
+
+def test_first_call_under_capture(device):
+    """A plan's first calls can be captured: they allocate nothing, and the
+    replay gives the bits of a call outside the capture."""
+    import torch
+    lmax, nlat, nphi, batch = 63, 96, 192, 16
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi))
+    q = torch.from_numpy(np.stack([spectrum(lmax, lmax, k) for k in range(batch)])).cuda()
+    fm = torch.zeros(2, batch, (lmax + 1) * nlat * 2, device="cuda")
+    out = torch.zeros(2, batch, q.shape[1], device="cuda")
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        plan.stage_dev("legSynth", q.data_ptr(), fm[0].data_ptr(), batch, stream.cuda_stream)
+        plan.stage_dev("legAnalys", fm[0].data_ptr(), out[0].data_ptr(), batch, stream.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    plan.stage_dev("legSynth", q.data_ptr(), fm[1].data_ptr(), batch)
+    plan.stage_dev("legAnalys", fm[0].data_ptr(), out[1].data_ptr(), batch)
+    device.sync()
+    assert torch.equal(fm[0], fm[1]) and torch.equal(out[0], out[1])
+    plan.destroy()
+
+
+def test_model_of_many_instances(device, parity):
+    """A batched FP32 model (the update in the epilogue of the products)
+    against the oracle and the launches it counts."""
+    lmax, nlat, nphi, batch, steps = 63, 96, 192, 9, 20
+    model = mModelByKey("schnakenberg")
+    p = defaultParams(model)
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi))
+    gpu = GpuModel.create(device, plan, model.source, [k.key for k in model.params], model.state,
+                          model.species, batch)
+    sets = [dict(p, D1=p["D1"] * (1 + 0.1 * k)) for k in range(batch)]
+    gpu.setParams(sets)
+    assert gpu.counts("step") == (5, 3)
+    gpu.init(np.concatenate([seededNoise(nlat * nphi, model.seedAmp, 1 + k) for k in range(batch)]))
+    st0 = [gpu.read(s) for s in model.state]
+    gpu.step(steps)
+    st = [gpu.read(s) for s in model.state]
+    ref = O.ShtReference(lmax, lmax, nlat, nphi)
+    for k in (0, batch - 1):
+        prm = [np.float32(sets[k][x.key]) for x in model.params]
+        want = ref.model_step("schnakenberg", prm, np.stack([s[k] for s in st0]).astype(np.float64), steps)
+        for i, name in enumerate(model.state):
+            parity(f"batched fp32 schnakenberg lmax63 {steps} steps inst{k} {name}",
+                   O.rel_l2(st[i][k], want[i]), 1e-4)
+    gpu.destroy()
+    plan.destroy()

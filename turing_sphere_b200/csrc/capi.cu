@@ -80,7 +80,7 @@ bool fft_radices(int nphi, TsFftTab &ft) {
 void plan_free(ts_plan p) {
   for (void *q : {(void *)p->d_x64, (void *)p->d_w64, (void *)p->d_ab64, (void *)p->d_amm64,
                   (void *)p->d_ct, (void *)p->d_st, (void *)p->d_wq, (void *)p->d_amm,
-                  (void *)p->d_ab, (void *)p->d_tw})
+                  (void *)p->d_ab, (void *)p->d_tw, (void *)p->lg_tab})
     if (q) cudaFree(q);
   p->fm.release();
   p->stage_q.release();

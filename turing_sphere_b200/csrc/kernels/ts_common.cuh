@@ -104,6 +104,15 @@ struct TsFftTab {
   int radix[16];
 };
 
+// A table of Legendre values of the batched FP32 products (see leg_gemm.cuh):
+// nhp padded latitudes; onset[m nhp + lat] is l - m of the first value that is
+// not zero.
+struct TsLegGemmTab {
+  const float *tab;
+  const int *onset;
+  int nhp;
+};
+
 // Tensor-core Legendre tables of a plan (see leg_tc.cuh).
 struct TsTcTab {
   const char *synth;        // synthesis image

@@ -59,6 +59,7 @@ struct Stage {
   int lb = 0, F = 1, K = 1, W = 1, per_cta = 1;
   int threads = 0;    // phase: threads per CTA (two-phase FFT: P*R, lb = R rows)
   bool wimg = false;  // tensor-core plan: the phase writes the W image itself
+  TsLgShape lg{};     // LegAnalys of a batch on an FP32 plan: the products' shape (ncol 0: recurrence)
   size_t smem = 0;
   // SpecEW: the variant that takes four consecutive coefficients per thread
   // (float4 loads and stores; used when every array and stride allows it)
@@ -209,6 +210,7 @@ struct ts_model_s {
   std::vector<StepGraph> graphs;
   bool use_graphs = true;
   int eager_left = 2;  // steps run eagerly first: every lazily grown buffer exists after them
+  bool host_only = false;  // ts_model_check: there is no device
   Adjoint adj;
 };
 
@@ -570,7 +572,63 @@ void schedule(ts_model m, Program &P, bool is_step) {
         throw tsm::CompileError{"too many analys outputs per instance for the tensor-core path",
                                 -1, -1, f.name};
     } else {
-      ts_analys_shape(p, m->batch * st.nana, st.nana, &st.F, &st.K, &st.W, &st.per_cta);
+      if (ts_lg_use(p, m->batch * st.nana, true) && (m->host_only || p->lg_tab)) {
+        ts_lg_analys_shape(p, m->batch * st.nana, st.nana, &st.lg);
+        st.per_cta = st.lg.per_cta;
+      } else {
+        ts_analys_shape(p, m->batch * st.nana, st.nana, &st.F, &st.K, &st.W, &st.per_cta);
+      }
+    }
+    if (st.lg.ncol) {
+      // epilogue of the products: one instance's NA analysed values of one
+      // coefficient, re and im, with the state read and written as pairs
+      Emitter ev{f, {}};
+      const std::string en = "TsEpi_" + ptag + std::to_string(tag++);
+      const size_t na = A.size();
+      std::ostringstream src;
+      src << "struct " << en << " {\n  static constexpr int NA = " << na << ";\n  TsSpecIO io;\n"
+          << "  static __device__ __forceinline__ void eval(const float *in, float *out, const float *prm) {\n"
+          << ev.scalars();
+      int k = 0;
+      for (int i : A) {
+        const int v = f.body[i].out;
+        src << "    const float v" << v << " = in[" << k++ << "];  // " << f.vars[v].name << "\n";
+        ev.name[v] = "v" + std::to_string(v);
+      }
+      for (int v : sin) {
+        src << "    const float v" << v << " = in[" << k++ << "];  // " << f.vars[v].name << "\n";
+        ev.name[v] = "v" + std::to_string(v);
+      }
+      for (int i : E) {
+        const auto &s = f.body[i];
+        src << "    const float v" << s.out << " = " << ev.e(s.expr) << ";  // " << f.vars[s.out].name
+            << "\n";
+        ev.name[s.out] = "v" + std::to_string(s.out);
+      }
+      for (size_t o = 0; o < sout.size(); o++) src << "    out[" << o << "] = v" << sout[o] << ";\n";
+      src << "  }\n  __device__ __forceinline__ void operator()(long inst, long lm, const float2 (&v)[NA]) "
+             "const {\n    const float *prm = io.prm + inst * io.nprm;\n"
+          << "    float re[" << na + sin.size() << "], im[" << na + sin.size() << "], ro["
+          << std::max<size_t>(sout.size(), 1) << "], io_[" << std::max<size_t>(sout.size(), 1) << "];\n";
+      for (size_t a = 0; a < na; a++)
+        src << "    re[" << a << "] = v[" << a << "].x, im[" << a << "] = v[" << a << "].y;\n";
+      for (size_t q = 0; q < sin.size(); q++)
+        src << "    const float2 x" << q << " = *reinterpret_cast<const float2 *>(io.sin[" << q
+            << "] + inst * io.sin_stride[" << q << "] + 2 * lm);\n    re[" << na + q << "] = x" << q
+            << ".x, im[" << na + q << "] = x" << q << ".y;\n";
+      src << "    eval(re, ro, prm);\n    eval(im, io_, prm);\n";
+      for (size_t o = 0; o < sout.size(); o++)
+        src << "    *reinterpret_cast<float2 *>(io.sout[" << o << "] + inst * io.sout_stride[" << o
+            << "] + 2 * lm) = make_float2(ro[" << o << "], io_[" << o << "]);\n";
+      src << "  }\n};\n";
+      st.expr = "ts_leg_analys_gemm<" + std::to_string(st.lg.ncol) + ", " + en + ">";
+      st.label = "legana  " + std::to_string(na) + " field(s), " + std::to_string(E.size()) +
+                 " spectral statement(s) fused";
+      st.src = src.str();
+      P.stages.push_back(st);
+      for (int i : E) done[i] = true;
+      for (int v : sout) avail[v] = true;
+      continue;
     }
     Emitter em{f, {}};
     const std::string en = "TsEpi_" + ptag + std::to_string(tag++);
@@ -666,7 +724,7 @@ std::vector<char> nvrtc_cubin(const std::string &code, const std::vector<std::st
 std::vector<char> build_cubin(ts_model m, std::map<std::string, std::string> &lowered) {
   std::ostringstream src;
   src << "#include \"ts_common.cuh\"\n#include \"fft2.cuh\"\n#include \"fourier.cuh\"\n#include \"leg_f32.cuh\"\n"
-      << "#include \"leg_tc.cuh\"\n";
+      << "#include \"leg_tc.cuh\"\n#include \"leg_gemm.cuh\"\n";
   for (auto &P : m->prog)
     for (auto &s : P.stages) src << stage_source(s);
   std::vector<std::string> exprs;
@@ -811,7 +869,12 @@ void run_program(ts_model m, Program &P, cudaStream_t st) {
         long gs = field;
         int nfields = B * s.nana;
         int per_cta = s.per_cta;
-        if (p->precision != TS_PREC_FP32) {
+        if (s.lg.ncol) {
+          TsLegGemmTab tab = p->lg_ana;
+          void *args[] = {&leg, &tab, &g, &gs, &epi, &nfields, &per_cta};
+          TS_CUDA(cudaLaunchKernel((const void *)s.kern, dim3(s.lg.grid[0], s.lg.grid[1], s.lg.grid[2]),
+                                   dim3(s.lg.threads), args, s.smem, st));
+        } else if (p->precision != TS_PREC_FP32) {
           TsTcTab tc = ts_tc_tab(p);
           int S = ts_tc_analys_stages(p);
           int nmax = ts_tc_analys_nmax(p);
@@ -868,7 +931,8 @@ void finish_shapes(ts_model m) {
         const int nrows = s.nsyn + s.nana + 1;
         if (!s.threads) s.lb = ts_fourier_lb(p, m->batch, nrows, &s.smem);
       } else if (s.kind == Stage::LegAnalys) {
-        s.smem = p->precision != TS_PREC_FP32 ? ts_tc_analys_smem(p) : ts_analys_smem(p, s.F, s.W);
+        s.smem = s.lg.ncol ? s.lg.smem
+                 : p->precision != TS_PREC_FP32 ? ts_tc_analys_smem(p) : ts_analys_smem(p, s.F, s.W);
       }
     }
 }
@@ -1895,6 +1959,7 @@ int ts_model_check(int lmax, int mmax, int nlat, int nphi, const char *source,
     plan.fft.mmax = mmax;
     plan.fft.nlat = nlat;
     mod.ctx = &ctx;
+    mod.host_only = true;
     mod.plan = &plan;
     mod.batch = batch;
     mod.source = source;

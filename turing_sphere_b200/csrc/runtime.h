@@ -112,6 +112,10 @@ struct ts_plan_s {
   TsFftTab fft{};
   // scratch: fm intermediate, host-call staging, adjoint scalings
   ts_dbuf fm, stage_q, stage_s, stage_q2, adj_grid, adj_spec;
+  // FP32 Legendre products (leg_gemm.cu): the tables of Legendre values of the
+  // two directions (null: they do not fit, the recurrence kernels run)
+  float *lg_tab = nullptr;
+  TsLegGemmTab lg_syn{}, lg_ana{};
   // tensor-core tables (precision != FP32)
   void *tc = nullptr;
   // kernel shapes: 0 = default (or TS_TC_NL / TS_TC_LTL); set by the autotuner
@@ -149,6 +153,23 @@ void ts_launch_leg_synth_fields(ts_plan p, const TsFields &q, float2 *fm, long f
 // the FP32 on-the-fly recurrence whatever the plan's precision (allocates nothing)
 void ts_launch_leg_synth_plain(ts_plan p, const TsFields &q, float2 *fm, long fm_stride,
                                int nfields, cudaStream_t s);
+// the same as FP32 products with a table of Legendre values (leg_gemm.cu):
+// ts_lg_use says by the sizes whether nf fields are better off with them; the
+// launchers return false, having done nothing, where it says no or the plan
+// has no table
+void ts_lg_init(ts_plan p);
+bool ts_lg_use(ts_plan p, int nf, bool analysis);
+bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fm_stride,
+                              int nfields, cudaStream_t s);
+bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *g, long g_stride, float2 *q, long q_stride,
+                               int nfields, cudaStream_t s);
+// launch shape of the analysis of nf fields in whole instances of na
+struct TsLgShape {
+  int ncol, per_cta, threads;
+  size_t smem;
+  unsigned grid[3];
+};
+void ts_lg_analys_shape(ts_plan p, int nf, int na, TsLgShape *sh);
 // analysis launch shape: fields per CTA F (template), latitudes per thread K,
 // warps W; groups = fields handled per CTA (a multiple of `per_inst`)
 void ts_analys_shape(ts_plan p, int nfields, int per_inst, int *F, int *K, int *W, int *per_cta);

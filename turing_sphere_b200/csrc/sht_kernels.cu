@@ -126,6 +126,18 @@ void ts_init_tables(ts_plan p) {
       p->d_st, p->d_wq, p->d_ab, p->d_amm);
   TS_CUDA(cudaGetLastError());
 
+  p->leg.ct = p->d_ct;
+  p->leg.st = p->d_st;
+  p->leg.wq = p->d_wq;
+  p->leg.ab = p->d_ab;
+  p->leg.amm = p->d_amm;
+  p->leg.lmax = p->lmax;
+  p->leg.mmax = p->mmax;
+  p->leg.nlat = p->nlat;
+  p->leg.nh = p->nh;
+  p->fft.tw = p->d_tw;
+  ts_lg_init(p);
+
   // twiddles e^{2 pi i k / nphi}: computed on the host in f64, as the
   // reference does (sht.ts:200-205), then rounded to float
   std::vector<float2> tw(p->nphi);
@@ -139,17 +151,6 @@ void ts_init_tables(ts_plan p) {
   TS_CUDA(cudaMemcpyAsync(p->h_x.data(), p->d_x64, sizeof(double) * nlat, cudaMemcpyDeviceToHost, s));
   TS_CUDA(cudaMemcpyAsync(p->h_w.data(), p->d_w64, sizeof(double) * nlat, cudaMemcpyDeviceToHost, s));
   TS_CUDA(cudaStreamSynchronize(s));
-
-  p->leg.ct = p->d_ct;
-  p->leg.st = p->d_st;
-  p->leg.wq = p->d_wq;
-  p->leg.ab = p->d_ab;
-  p->leg.amm = p->d_amm;
-  p->leg.lmax = p->lmax;
-  p->leg.mmax = p->mmax;
-  p->leg.nlat = p->nlat;
-  p->leg.nh = p->nh;
-  p->fft.tw = p->d_tw;
 }
 
 // ------------------------------------------------------------- DFT stage
@@ -308,6 +309,7 @@ void ts_kernel_attrs_once(ts_ctx ctx) {
 void ts_launch_leg_synth_fields(ts_plan p, const TsFields &q, float2 *fm, long fs, int nf,
                                 cudaStream_t s) {
   if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, q, fm, fs, nf, s);
+  if (ts_launch_leg_synth_gemm(p, q, fm, fs, nf, s)) return;
   ts_launch_leg_synth_plain(p, q, fm, fs, nf, s);
 }
 
@@ -365,13 +367,12 @@ int ts_fourier_lb(ts_plan p, int nblocks_y, int nrows, size_t *smem) {
 
 void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long fs, int nf,
                          cudaStream_t s) {
-  if (p->precision != TS_PREC_FP32) {
-    TsFields qf{};
-    qf.base[0] = q;
-    qf.inst_stride[0] = qs;
-    qf.nper = 1;
-    return ts_launch_leg_synth_tc(p, qf, fm, fs, nf, s);
-  }
+  TsFields qf{};
+  qf.base[0] = q;
+  qf.inst_stride[0] = qs;
+  qf.nper = 1;
+  if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, qf, fm, fs, nf, s);
+  if (ts_launch_leg_synth_gemm(p, qf, fm, fs, nf, s)) return;
   if (nf >= 8) return leg_synth_t<8>(p, q, qs, fm, fs, nf, s);
   if (nf >= 4) return leg_synth_t<4>(p, q, qs, fm, fs, nf, s);
   if (nf >= 2) return leg_synth_t<2>(p, q, qs, fm, fs, nf, s);
@@ -381,6 +382,7 @@ void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long f
 void ts_launch_leg_analys(ts_plan p, const float2 *g, long gs, float2 *q, long qs, int nf,
                           cudaStream_t s) {
   if (p->precision != TS_PREC_FP32) return ts_launch_leg_analys_tc(p, g, gs, q, qs, nf, s);
+  if (ts_launch_leg_analys_gemm(p, g, gs, q, qs, nf, s)) return;
   int K, W;
   pick_kw(p->nh, K, W);
   // registers hold K*F complex pairs of weighted inputs: keep K*F <= 24
