@@ -109,3 +109,38 @@ def test_model_of_many_instances(device, parity):
                    O.rel_l2(st[i][k], want[i]), 1e-4)
     gpu.destroy()
     plan.destroy()
+
+
+# (lmax, mmax, nlat, nphi, batch): on a tensor-core plan the largest batches of
+# the products and the smallest of the contraction, on grids whose tables lie
+# on either side of 2 and 64 MB, with odd latitudes and mmax < lmax
+TC_CASES = [(63, 63, 96, 192, 48), (63, 63, 96, 192, 49), (100, 90, 151, 512, 16),
+            (100, 90, 151, 512, 17), (170, 150, 257, 512, 48), (170, 150, 257, 512, 65),
+            (255, 255, 384, 768, 1), (319, 319, 640, 1536, 33)]
+
+
+@pytest.mark.parametrize("lmax,mmax,nlat,nphi,batch", TC_CASES)
+def test_batches_of_a_tensor_core_plan(device, parity, lmax, mmax, nlat, nphi, batch):
+    """Every field of both routes against the f64 oracle's transform of the
+    first one (relative L2 <= 1e-5: the bar of both plans' transforms)."""
+    import torch
+    plan = ShtPlan.create(device, ShtConfig(lmax, mmax, nlat, nphi), {"precision": "tf32x3"})
+    ref = O.ShtReference(lmax, mmax, nlat, nphi)
+    scale = np.ldexp(np.float32(1), -(np.arange(batch) % 5)).astype(np.float32)[:, None]
+    q = spectrum(lmax, mmax, lmax + batch)
+    want = ref.synth(q.astype(np.float64))
+    g = want.astype(np.float32)
+    worst = [0.0, 0.0]
+    for k, (call, x, y) in enumerate(((plan.synth_dev, q, want),
+                                      (plan.analys_dev, g, ref.analys(g.astype(np.float64))))):
+        src = torch.from_numpy(scale * x[None, :]).cuda()
+        dst = torch.empty(batch, y.size, device="cuda")
+        torch.cuda.synchronize()
+        call(src.data_ptr(), dst.data_ptr(), batch)
+        device.sync()
+        got = dst.cpu().numpy() / scale
+        worst[k] = max(O.rel_l2(got[f], y) for f in range(batch))
+    plan.status()
+    parity(f"tf32x3 lmax{lmax} mmax{mmax} nlat{nlat} B{batch} synth", worst[0], TOL)
+    parity(f"tf32x3 lmax{lmax} mmax{mmax} nlat{nlat} B{batch} analys", worst[1], TOL)
+    plan.destroy()

@@ -3,8 +3,9 @@
 //   synthesis  F_par[lat, c] = sum_j P_par[j, lat] Q_par[j, c],   north = F_0 + F_1, south = F_0 - F_1
 //   analysis   Q_par[j, c]   = sum_lat P_par[lat, j] W_par[lat, c], W_0, W_1 = (G_north +- G_south) w
 // for one order m, degrees l = m + 2j + par, real columns c = 2 field + re|im.
-// The table (ts_leg_ptab_f32, written once per plan) holds what the on-the-fly
-// recurrence of leg_f32.cuh gives.  The recurrence kernels spend most of their
+// The table, written once per plan, holds what the on-the-fly recurrence of
+// leg_f32.cuh gives or, for the small batches of a tensor-core plan, the FP64
+// functions rounded to FP32.  The recurrence kernels spend most of their
 // time on 8-byte shared loads per two multiply-adds (synthesis) and on a
 // shuffle reduction per pair of degrees (analysis); these are bound by the
 // FP32 pipe.  At lmax 255 (384 latitudes), 256 fields: synthesis 364 -> 154
@@ -79,50 +80,49 @@ TS_DEV void ts_lg_cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ------------------------------------------------------------- FP32 table
+// ------------------------------------------------------------------ tables
 //
-// One thread per order and latitude: the recurrence of ts_leg_synth_f32, its
-// products and sums rounded as they are there (a synthesis by way of the table
-// gives the same bits); zeros in the padding.  A value counts only once the running exponent is
-// zero: onset is the first l - m where it does (lmax + 1: never), so that the
-// products can leave out what is zero near the poles.  Coefficients past lmax
-// are read as zeros, which ends the recurrence without a test; the rescaling
-// tests run only while some latitude of the warp still carries an exponent.
-// The synthesis layout is written as it comes (16 degrees at a time, lanes on
-// consecutive latitudes), the analysis layout by way of shared memory, 32
-// degrees of a parity as one 128-byte line of a latitude.
-// grid = (nhp / 64, mmax + 1), 64 threads, 2 ts_lg_k16(lmax, 0, 0) + 4 float2 of shared memory.
-template <bool ANALYSIS>
-__global__ void __launch_bounds__(64)
-ts_leg_ptab_f32(TsLegTab t, TsLegGemmTab g, float *__restrict__ tab, int *__restrict__ onset) {
-  extern __shared__ __align__(16) float2 ts_smem_pt[];
-  constexpr int VP = 36;  // pitch: 16-byte rows, 8 lanes in distinct banks
-  __shared__ __align__(16) float sv[ANALYSIS ? 2 * 64 * VP : 4];
-  const int m = blockIdx.y, lat0 = blockIdx.x * 64, lat = lat0 + threadIdx.x;
-  const int K = t.lmax - m + 1, k0 = ts_lg_k16(t.lmax, m, 0), k1 = ts_lg_k16(t.lmax, m, 1);
-  const long base = ts_lm_base(t.lmax, m);
-  float2 *sab = ts_smem_pt;
-  for (int i = threadIdx.x; i < 2 * k0 + 4; i += blockDim.x)
-    sab[i] = i < K ? t.ab[base + i] : make_float2(0.f, 0.f);
-  __syncthreads();
-  const bool live = lat < t.nh;
-  const float ct = live ? t.ct[lat] : 0.f;
-  float y0 = 0.f, y1 = 0.f;
-  int ny = 0, first = live ? -1 : t.lmax + 1;
-  if (live) {
-    ts_sinpow(t.st[lat], m, y0, ny);
-    y0 *= t.amm[m];
-    y1 = sab[1].x * ct * y0;
+// One thread per order and latitude walks a recurrence over the degrees, 8
+// pairs (l - m = 2j, 2j + 1) at a time; zeros in the padding.  onset is the
+// first l - m with a value that is not zero (lmax + 1: none), so that the
+// products can leave out what is zero near the poles.  The synthesis layout is
+// written as it comes (16 degrees at a time, lanes on consecutive latitudes),
+// the analysis layout by way of shared memory, 32 degrees of a parity as one
+// 128-byte line of a latitude.
+// grid = (nhp / 64, mmax + 1), 64 threads, 2 ts_lg_k16(lmax, 0, 0) + 4
+// coefficient pairs of the recurrence's type in shared memory.
+
+// The recurrence of ts_leg_synth_f32, its products and sums rounded as they are
+// there (a synthesis by way of the table gives the same bits).  A value counts
+// only once the running exponent is zero.  Coefficients past lmax are read as
+// zeros, which ends the recurrence without a test; the rescaling tests run only
+// while some latitude of the warp still carries an exponent.
+struct TsLgRec32 {
+  using Pair = float2;
+  TsLegTab t;
+  float ct, y0, y1;
+  int ny, first;
+  TS_DEV explicit TsLgRec32(const TsLegTab &t_) : t(t_) {}
+  TS_DEV Pair coeff(long lm) const { return t.ab[lm]; }
+  TS_DEV void init(int m, int lat, const Pair *sab) {
+    const bool live = lat < t.nh;
+    ct = live ? t.ct[lat] : 0.f;
+    y0 = y1 = 0.f;
+    ny = 0;
+    first = live ? -1 : t.lmax + 1;
+    if (live) {
+      ts_sinpow(t.st[lat], m, y0, ny);
+      y0 *= t.amm[m];
+      y1 = sab[1].x * ct * y0;
+    }
   }
-  auto advance = [&](int i) {
+  TS_DEV void advance(const Pair *sab, int i) {
     const float4 a = *reinterpret_cast<const float4 *>(sab + i + 2);
     const float t0 = fmaf(__fmul_rn(a.x, ct), y1, __fmul_rn(a.y, y0));
     y1 = fmaf(a.w, y1, __fmul_rn(__fmul_rn(a.z, ct), t0));
     y0 = t0;
-  };
-  float *mt = tab + ts_lg_off(t.lmax, m) * g.nhp;
-  for (int j0 = 0; j0 < k0; j0 += 8) {
-    float v[2][8];
+  }
+  TS_DEV void next8(const Pair *sab, int j0, float (&v)[2][8]) {
     if (__any_sync(0xffffffffu, first < 0)) {
 #pragma unroll
       for (int u = 0; u < 8; u++) {
@@ -136,16 +136,90 @@ ts_leg_ptab_f32(TsLegTab t, TsLegGemmTab g, float *__restrict__ tab, int *__rest
         ny += up ? 1 : 0;
         y0 *= f;
         y1 *= f;
-        advance(i);
+        advance(sab, i);
       }
     } else {
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         v[0][u] = y0;
         v[1][u] = y1;
-        advance(2 * (j0 + u));
+        advance(sab, 2 * (j0 + u));
       }
     }
+  }
+};
+
+// The recurrence of the tensor-core tables in FP64 (a running pair scaled by
+// powers of 2^500), each value rounded once to FP32; values below 1e-15 before
+// the first larger one count as zero, as in the FP32 recurrence.
+struct TsLgRec64 {
+  using Pair = double2;
+  const double *x, *ab, *amm;
+  int lmax, nh;
+  double ct, y0, y1;
+  int e, first;
+  TS_DEV TsLgRec64(const double *x_, const double *ab_, const double *amm_, int lmax_, int nh_)
+      : x(x_), ab(ab_), amm(amm_), lmax(lmax_), nh(nh_) {}
+  TS_DEV Pair coeff(long lm) const { return make_double2(ab[2 * lm], ab[2 * lm + 1]); }
+  TS_DEV void init(int m, int lat, const Pair *sab) {
+    const bool live = lat < nh;
+    ct = live ? x[lat] : 0.0;
+    first = live ? -1 : lmax + 1;
+    e = 0;
+    y0 = y1 = 0.0;
+    if (!live) return;
+    const double st = sqrt(1.0 - ct * ct);
+    double y = 1.0;
+    for (int i = 0; i < m; i++) {
+      y *= st;
+      if (y < 0x1p-500) {
+        y *= 0x1p500;
+        e -= 500;
+      }
+    }
+    y0 = y * amm[m];
+    y1 = sab[1].x * ct * y0;
+  }
+  TS_DEV float value(double y, int i) {
+    const double p = e < -1100 ? 0.0 : e == 0 ? y : ldexp(y, e);
+    if (first < 0 && fabs(p) >= 1e-15) first = i;
+    return first < 0 ? 0.f : (float)p;
+  }
+  TS_DEV void next8(const Pair *sab, int j0, float (&v)[2][8]) {
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = 2 * (j0 + u);
+      v[0][u] = value(y0, i);
+      v[1][u] = value(y1, i + 1);
+      const double2 a0 = sab[i + 2], a1 = sab[i + 3];
+      y0 = a0.x * ct * y1 + a0.y * y0;
+      y1 = a1.x * ct * y0 + a1.y * y1;
+      if (fabs(y1) > 0x1p500) {
+        y0 *= 0x1p-500;
+        y1 *= 0x1p-500;
+        e += 500;
+      }
+    }
+  }
+};
+
+template <bool ANALYSIS, class Rec>
+TS_DEV void ts_lg_table(Rec rec, int lmax, int nhp, float *__restrict__ tab, int *__restrict__ onset) {
+  extern __shared__ __align__(16) char ts_smem_pt[];
+  using Pair = typename Rec::Pair;
+  constexpr int VP = 36;  // pitch: 16-byte rows, 8 lanes in distinct banks
+  __shared__ __align__(16) float sv[ANALYSIS ? 2 * 64 * VP : 4];
+  const int m = blockIdx.y, lat0 = blockIdx.x * 64, lat = lat0 + threadIdx.x;
+  const int K = lmax - m + 1, k0 = ts_lg_k16(lmax, m, 0), k1 = ts_lg_k16(lmax, m, 1);
+  const long base = ts_lm_base(lmax, m);
+  Pair *sab = reinterpret_cast<Pair *>(ts_smem_pt);
+  for (int i = threadIdx.x; i < 2 * k0 + 4; i += blockDim.x) sab[i] = i < K ? rec.coeff(base + i) : Pair{};
+  __syncthreads();
+  rec.init(m, lat, sab);
+  float *mt = tab + ts_lg_off(lmax, m) * nhp;
+  for (int j0 = 0; j0 < k0; j0 += 8) {
+    float v[2][8];
+    rec.next8(sab, j0, v);
     if constexpr (ANALYSIS) {
 #pragma unroll
       for (int par = 0; par < 2; par++) {
@@ -159,7 +233,7 @@ ts_leg_ptab_f32(TsLegTab t, TsLegGemmTab g, float *__restrict__ tab, int *__rest
 #pragma unroll
         for (int par = 0; par < 2; par++) {
           const int kp = par ? k1 : k0;
-          float *dst = mt + (par ? (long)k0 * g.nhp : 0) + jj;
+          float *dst = mt + (par ? (long)k0 * nhp : 0) + jj;
           if (jj < kp)
 #pragma unroll
             for (int u = 0; u < 8; u++)
@@ -172,13 +246,26 @@ ts_leg_ptab_f32(TsLegTab t, TsLegGemmTab g, float *__restrict__ tab, int *__rest
 #pragma unroll
       for (int par = 0; par < 2; par++) {
         if (j0 >= (par ? k1 : k0)) continue;
-        float *dst = mt + (long)((par ? k0 : 0) + j0) * g.nhp + lat;
+        float *dst = mt + (long)((par ? k0 : 0) + j0) * nhp + lat;
 #pragma unroll
-        for (int u = 0; u < 8; u++) dst[(long)u * g.nhp] = v[par][u];
+        for (int u = 0; u < 8; u++) dst[(long)u * nhp] = v[par][u];
       }
     }
   }
-  onset[(long)m * g.nhp + lat] = first < 0 ? t.lmax + 1 : first;
+  onset[(long)m * nhp + lat] = rec.first < 0 ? lmax + 1 : rec.first;
+}
+
+template <bool ANALYSIS>
+__global__ void __launch_bounds__(64)
+ts_leg_ptab_f32(TsLegTab t, int nhp, float *__restrict__ tab, int *__restrict__ onset) {
+  ts_lg_table<ANALYSIS>(TsLgRec32(t), t.lmax, nhp, tab, onset);
+}
+
+template <bool ANALYSIS>
+__global__ void __launch_bounds__(64)
+ts_leg_ptab_f64(const double *x, const double *ab, const double *amm, int lmax, int nh, int nhp,
+                float *__restrict__ tab, int *__restrict__ onset) {
+  ts_lg_table<ANALYSIS>(TsLgRec64(x, ab, amm, lmax, nh), lmax, nhp, tab, onset);
 }
 
 // ------------------------------------------------------------ shared parts

@@ -14,7 +14,24 @@ size_t lg_bytes(ts_plan p) {
   return sizeof(float) * lg_floats(p) + sizeof(int) * (size_t)(p->mmax + 1) * lg_nhp(p);
 }
 bool lg_fits(ts_plan p) {
-  return p->precision == TS_PREC_FP32 && p->lmax <= 2047 && lg_bytes(p) <= (size_t)512 << 20;
+  if (p->precision == TS_PREC_FP32) return p->lmax <= 2047 && lg_bytes(p) <= (size_t)512 << 20;
+  return p->lmax <= 1535 && lg_bytes(p) <= (size_t)2 << 30;
+}
+
+// the plan's table, made by the first call that wants it on a tensor-core plan
+// (whose large batches never do): false when there is none and it cannot be
+// made now, because the stream is being captured or memory is short
+bool lg_ready(ts_plan p, cudaStream_t s) {
+  if (p->lg_tab) return true;
+  if (p->precision == TS_PREC_FP32) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  ts_lg_init(p, s);
+  if (p->lg_tab) TS_CUDA(cudaStreamSynchronize(s));  // later calls may come on other streams
+  return p->lg_tab != nullptr;
 }
 
 // columns of a tile (2 per field) with the least work for nf fields in whole
@@ -69,14 +86,33 @@ void analys_t(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, const
 // one or two fields' synthesis where the table comes from HBM (over 64 MB).
 // Above 512 MB the table is not made, nor above lmax 2047 (the recurrence
 // coefficients of an order are held in shared memory).
+//
+// On tensor-core plans the contraction works in blocks of 64 fields, so a small
+// batch is mostly padding there; the products read half the table bytes and
+// round the table once (error against 64 bits at lmax 511: 4.4e-7, contraction
+// 4.9e-6).  Whole transforms (us, contraction | products; 3/2 grids):
+//   synthesis  lmax 63: 1 field 19.3 | 12.2, 64: 21.6 | 13.6;  lmax 127: 1: 24.8 | 12.4, 64: 32 | 27.5;
+//              lmax 255: 1: 42 | 18.7, 16: 51 | 28, 48: 67 | 61, 64: 76 | 76;  lmax 511: 1: 148 | 63,
+//              32: 241 | 225, 48: 287 | 343;  lmax 1023: 1: 759 | 343, 16: 961 | 660, 24: 1064 | 1132
+//   analysis   lmax 63: 1: 13.2 | 12.4, 48: 16.5 | 12.8;  lmax 127: 1: 18.7 | 12.9, 16: 18.7 | 17.1,
+//              24: 19.7 | 22.8;  lmax 255: 1: 35 | 24, 16: 43 | 35, 24: 48 | 55;  lmax 1023: 16: 869 | 677,
+//              24: 966 | 1195
+// so the line lies at 16 fields, or for the synthesis at 48 where the table
+// stays in the L2 and 32 up to 256 MB, and for the smallest analyses at 48.
+// No table above 2 GB or lmax 1535.
 bool ts_lg_use(ts_plan p, int nf, bool analysis) {
   const size_t bytes = lg_bytes(p);
   if (!lg_fits(p)) return false;
+  if (p->precision != TS_PREC_FP32) {
+    if (ts_tc_stalled(p)) return false;  // the test hook is about the tensor-core kernels
+    if (analysis) return nf <= (bytes < (size_t)2 << 20 ? 48 : 16);
+    return nf <= (bytes <= (size_t)64 << 20 ? 48 : bytes <= (size_t)256 << 20 ? 32 : 16);
+  }
   if (bytes < (size_t)384 << 10) return nf >= 8;
   return analysis || nf >= 3 || bytes <= (size_t)64 << 20;
 }
 
-void ts_lg_init(ts_plan p) {
+void ts_lg_init(ts_plan p, cudaStream_t s) {
   if (!lg_fits(p)) return;
   const size_t n = lg_floats(p), no = (size_t)(p->mmax + 1) * lg_nhp(p);
   float *tab = nullptr;
@@ -86,20 +122,29 @@ void ts_lg_init(ts_plan p) {
   }
   p->lg_tab = tab;
   int *onset = (int *)(tab + 2 * n);
-  p->lg_syn = TsLegGemmTab{tab, onset, lg_nhp(p)};
-  p->lg_ana = TsLegGemmTab{tab + n, onset, lg_nhp(p)};
-  const size_t smem = sizeof(float2) * (2 * lg_k16(p->lmax, 0, 0) + 4);
-  const dim3 grid(lg_nhp(p) / 64, p->mmax + 1);
-  cudaStream_t s = p->ctx->stream;
-  ts_leg_ptab_f32<false><<<grid, 64, smem, s>>>(p->leg, p->lg_syn, tab, onset);
-  TS_CUDA(cudaGetLastError());
-  ts_leg_ptab_f32<true><<<grid, 64, smem, s>>>(p->leg, p->lg_ana, tab + n, onset);
+  const int nhp = lg_nhp(p), pairs = 2 * lg_k16(p->lmax, 0, 0) + 4;
+  p->lg_syn = TsLegGemmTab{tab, onset, nhp};
+  p->lg_ana = TsLegGemmTab{tab + n, onset, nhp};
+  const dim3 grid(nhp / 64, p->mmax + 1);
+  if (p->precision == TS_PREC_FP32) {
+    const size_t smem = sizeof(float2) * pairs;
+    ts_leg_ptab_f32<false><<<grid, 64, smem, s>>>(p->leg, nhp, tab, onset);
+    TS_CUDA(cudaGetLastError());
+    ts_leg_ptab_f32<true><<<grid, 64, smem, s>>>(p->leg, nhp, tab + n, onset);
+  } else {
+    const size_t smem = sizeof(double2) * pairs;
+    ts_leg_ptab_f64<false><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
+                                                  tab, onset);
+    TS_CUDA(cudaGetLastError());
+    ts_leg_ptab_f64<true><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
+                                                 tab + n, onset);
+  }
   TS_CUDA(cudaGetLastError());
 }
 
 bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fs, int nf,
                               cudaStream_t s) {
-  if (!p->lg_tab || !ts_lg_use(p, nf, false)) return false;
+  if (!ts_lg_use(p, nf, false) || !lg_ready(p, s)) return false;
   const TsLegGemmTab &g = p->lg_syn;
   switch (lg_ncol(nf, 1)) {
     case 64: synth_t<64>(p, g, q, fm, fs, nf, s); break;
@@ -112,7 +157,7 @@ bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fs,
 
 bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *gm, long gs, float2 *out, long os, int nf,
                                cudaStream_t s) {
-  if (!p->lg_tab || !ts_lg_use(p, nf, true)) return false;
+  if (!ts_lg_use(p, nf, true) || !lg_ready(p, s)) return false;
   const TsLegGemmTab &g = p->lg_ana;
   TsLgStore st{};
   st.base[0] = out;
@@ -126,6 +171,8 @@ bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *gm, long gs, float2 *out
   TS_CUDA(cudaGetLastError());
   return true;
 }
+
+bool ts_lg_prepare(ts_plan p, cudaStream_t s) { return lg_ready(p, s); }
 
 void ts_lg_analys_shape(ts_plan p, int nf, int na, TsLgShape *sh) {
   sh->ncol = lg_ncol(nf, na);

@@ -451,6 +451,7 @@ void schedule(ts_model m, Program &P, bool is_step) {
     }
     if ((int)gin.size() > TS_MAXIO || (int)gout.size() > TS_MAXIO || (int)S.size() > TS_MAXIO)
       throw tsm::CompileError{"too many grid fields in one phase (limit 8)", -1, -1, f.name};
+    bool lg = false;  // the phase's analysis runs as the FP32 products
     if (!S.empty()) {
       Stage st;
       st.kind = Stage::LegSynth;
@@ -499,7 +500,9 @@ void schedule(ts_model m, Program &P, bool is_step) {
       int fP = 0, fQ = 0, fR = 0;
       const int nb = std::max<int>({(int)S.size(), (int)A.size(), 1});
       if (ts_f2_phase_shape(p, &fP, &fQ)) fR = ts_f2_phase_rows(p, nb, m->batch, &st.smem);
-      const bool tcw = p->precision != TS_PREC_FP32 && fR && !A.empty();
+      lg = !A.empty() && ts_lg_use(p, m->batch * (int)A.size(), true) &&
+           (m->host_only || ts_lg_prepare(p, m->ctx->stream));
+      const bool tcw = p->precision != TS_PREC_FP32 && !lg && fR && !A.empty();
       if (fR) {
         st.expr = "ts_f2_phase<" + pn + ", " + std::to_string(fP) + ", " + std::to_string(fQ) +
                   ", " + std::to_string(fR) + ", " + (tcw ? "true" : "false") + ">";
@@ -529,7 +532,7 @@ void schedule(ts_model m, Program &P, bool is_step) {
     // 64-field block for one coefficient; with many instances that loop of
     // dependent state loads is latency-bound, so the analysis only stores and
     // the spectral statements run as a coalesced element-wise stage (A).
-    const bool fuse_epi = p->precision == TS_PREC_FP32 || m->batch * (long)A.size() <= 16;
+    const bool fuse_epi = p->precision == TS_PREC_FP32 || lg || m->batch * (long)A.size() <= 16;
     for (size_t i = 0; i < f.body.size() && fuse_epi; i++) {
       const auto &s = f.body[i];
       if (done[i] || s.kind != tsm::Stmt::Elementwise || f.vars[s.out].dom != Dom::Spec) continue;
@@ -565,14 +568,14 @@ void schedule(ts_model m, Program &P, bool is_step) {
     st.wimg = P.stages.back().kind == Stage::Phase && P.stages.back().wimg;
     for (int v : sin) st.in.push_back(ref[v]);
     for (int v : sout) st.out.push_back(ref[v]);
-    const bool tc = p->precision != TS_PREC_FP32;
+    const bool tc = p->precision != TS_PREC_FP32 && !lg;
     if (tc) {
       st.per_cta = st.nana * (TS_TC_FIELDS / st.nana);  // whole instances per 64-field block
       if (st.per_cta == 0)
         throw tsm::CompileError{"too many analys outputs per instance for the tensor-core path",
                                 -1, -1, f.name};
     } else {
-      if (ts_lg_use(p, m->batch * st.nana, true) && (m->host_only || p->lg_tab)) {
+      if (lg) {
         ts_lg_analys_shape(p, m->batch * st.nana, st.nana, &st.lg);
         st.per_cta = st.lg.per_cta;
       } else {
@@ -822,9 +825,9 @@ void run_program(ts_model m, Program &P, cudaStream_t st) {
           q.inst_stride[i] = stride / 2;
         }
         q.nper = s.nsyn;
-        if (p->precision != TS_PREC_FP32)
+        if (p->precision != TS_PREC_FP32 && !ts_launch_leg_synth_gemm(p, q, fm, field, B * s.nsyn, st))
           ts_launch_leg_synth_tc(p, q, fm, field, B * s.nsyn, st, &m->qimg);
-        else
+        else if (p->precision == TS_PREC_FP32)
           ts_launch_leg_synth_fields(p, q, fm, field, B * s.nsyn, st);
         break;
       }
@@ -1465,12 +1468,19 @@ int ts_model_compile(ts_plan plan, const char *source, const char *const *state,
       size_t wb = 0;
       for (auto &P : m->prog)
         for (auto &st : P.stages)
-          if (st.kind == Stage::LegAnalys)
+          if (st.kind == Stage::LegAnalys && !st.lg.ncol)
             wb = std::max(wb, ts_tc_wimg_bytes(plan, batch * st.nana, st.per_cta));
       m->wimg.ensure(std::max<size_t>(wb, 16));
       TS_CUDA(cudaMemset(m->wimg.p, 0, m->wimg.cap));
-      m->qimg.ensure(ts_tc_qimg_bytes(plan, batch * nsyn));
-      TS_CUDA(cudaMemset(m->qimg.p, 0, m->qimg.cap));
+      bool image = false;  // some synthesis is the contraction
+      for (auto &P : m->prog)
+        for (auto &st : P.stages)
+          image = image || (st.kind == Stage::LegSynth &&
+                            !(ts_lg_use(plan, batch * st.nsyn, false) && ts_lg_prepare(plan, ctx->stream)));
+      if (image) {
+        m->qimg.ensure(ts_tc_qimg_bytes(plan, batch * nsyn));
+        TS_CUDA(cudaMemset(m->qimg.p, 0, m->qimg.cap));
+      }
     }
     m->stash.ensure(sizeof(float) * 2 * nlm * batch * nstate);
     m->h_prm.assign((size_t)std::max(nparams, 1) * batch, 0.0f);
@@ -1909,11 +1919,15 @@ int ts_model_source(ts_model m, char *buf, size_t cap) {
 
 namespace {
 // CUDA kernel launches of one call of a program: on a tensor-core plan a
-// Legendre synthesis stage is two (the operand relayout, then the tcgen05
+// large batch's Legendre synthesis stage is two (the operand relayout, then the tcgen05
 // contraction)
-int kernel_launches(ts_plan p, const Program &P) {
+int kernel_launches(ts_model m, const Program &P) {
   int n = 0;
-  for (auto &s : P.stages) n += s.kind == Stage::LegSynth && p->precision != TS_PREC_FP32 ? 2 : 1;
+  for (auto &s : P.stages)
+    n += s.kind == Stage::LegSynth && m->plan->precision != TS_PREC_FP32 &&
+                 !ts_lg_use(m->plan, m->batch * s.nsyn, false)
+             ? 2
+             : 1;
   return n;
 }
 }  // namespace
@@ -1922,7 +1936,7 @@ int ts_model_counts(ts_model m, int which, int *kernels, int *launches) {
   TSM_BEGIN(m)
   TS_REQUIRE(which == 0 || which == 1, TS_ERR_INVALID, "which: 0 = init, 1 = step");
   if (kernels) *kernels = tsm::count_kernels(m->prog[which].fn);
-  if (launches) *launches = kernel_launches(m->plan, m->prog[which]);
+  if (launches) *launches = kernel_launches(m, m->prog[which]);
   TSM_END
 }
 
@@ -1986,7 +2000,7 @@ int ts_model_check(int lmax, int mmax, int nlat, int nphi, const char *source,
                describe_program(mod.prog[1]).c_str());
     }
     if (kernels) *kernels = tsm::count_kernels(mod.prog[1].fn);
-    if (launches) *launches = kernel_launches(&plan, mod.prog[1]);
+    if (launches) *launches = kernel_launches(&mod, mod.prog[1]);
     return TS_OK;
   } catch (const ts_exc &e) {
     if (err && err->message[0] == 0) snprintf(err->message, sizeof err->message, "%s", e.msg.c_str());

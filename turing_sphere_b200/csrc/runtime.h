@@ -113,7 +113,7 @@ struct ts_plan_s {
   // scratch: fm intermediate, host-call staging, adjoint scalings
   ts_dbuf fm, stage_q, stage_s, stage_q2, adj_grid, adj_spec;
   // FP32 Legendre products (leg_gemm.cu): the tables of Legendre values of the
-  // two directions (null: they do not fit, the recurrence kernels run)
+  // two directions (null: not made, or they do not fit)
   float *lg_tab = nullptr;
   TsLegGemmTab lg_syn{}, lg_ana{};
   // tensor-core tables (precision != FP32)
@@ -157,7 +157,8 @@ void ts_launch_leg_synth_plain(ts_plan p, const TsFields &q, float2 *fm, long fm
 // ts_lg_use says by the sizes whether nf fields are better off with them; the
 // launchers return false, having done nothing, where it says no or the plan
 // has no table
-void ts_lg_init(ts_plan p);
+void ts_lg_init(ts_plan p, cudaStream_t s);
+bool ts_lg_prepare(ts_plan p, cudaStream_t s);  // the table is there (made now if it can be)
 bool ts_lg_use(ts_plan p, int nf, bool analysis);
 bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fm_stride,
                               int nfields, cudaStream_t s);
@@ -207,6 +208,7 @@ struct TsTcGeom {
 };
 TsTcGeom ts_tc_geom(ts_plan p);
 void ts_tc_set_fault(ts_plan p, int stall_copies, unsigned wait_limit);
+bool ts_tc_stalled(ts_plan p);
 // tiles / chunks the tensor-core polar skip drops
 void ts_tc_skip_counts(ts_plan p, int *tiles, int *chunks);
 // per (32-latitude chunk, parity): the order m from which the W image's chunk

@@ -136,7 +136,7 @@ void ts_init_tables(ts_plan p) {
   p->leg.nlat = p->nlat;
   p->leg.nh = p->nh;
   p->fft.tw = p->d_tw;
-  ts_lg_init(p);
+  if (p->precision == TS_PREC_FP32) ts_lg_init(p, s);
 
   // twiddles e^{2 pi i k / nphi}: computed on the host in f64, as the
   // reference does (sht.ts:200-205), then rounded to float
@@ -308,8 +308,8 @@ void ts_kernel_attrs_once(ts_ctx ctx) {
 
 void ts_launch_leg_synth_fields(ts_plan p, const TsFields &q, float2 *fm, long fs, int nf,
                                 cudaStream_t s) {
-  if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, q, fm, fs, nf, s);
   if (ts_launch_leg_synth_gemm(p, q, fm, fs, nf, s)) return;
+  if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, q, fm, fs, nf, s);
   ts_launch_leg_synth_plain(p, q, fm, fs, nf, s);
 }
 
@@ -371,8 +371,8 @@ void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long f
   qf.base[0] = q;
   qf.inst_stride[0] = qs;
   qf.nper = 1;
-  if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, qf, fm, fs, nf, s);
   if (ts_launch_leg_synth_gemm(p, qf, fm, fs, nf, s)) return;
+  if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, qf, fm, fs, nf, s);
   if (nf >= 8) return leg_synth_t<8>(p, q, qs, fm, fs, nf, s);
   if (nf >= 4) return leg_synth_t<4>(p, q, qs, fm, fs, nf, s);
   if (nf >= 2) return leg_synth_t<2>(p, q, qs, fm, fs, nf, s);
@@ -381,8 +381,8 @@ void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long f
 
 void ts_launch_leg_analys(ts_plan p, const float2 *g, long gs, float2 *q, long qs, int nf,
                           cudaStream_t s) {
-  if (p->precision != TS_PREC_FP32) return ts_launch_leg_analys_tc(p, g, gs, q, qs, nf, s);
   if (ts_launch_leg_analys_gemm(p, g, gs, q, qs, nf, s)) return;
+  if (p->precision != TS_PREC_FP32) return ts_launch_leg_analys_tc(p, g, gs, q, qs, nf, s);
   int K, W;
   pick_kw(p->nh, K, W);
   // registers hold K*F complex pairs of weighted inputs: keep K*F <= 24

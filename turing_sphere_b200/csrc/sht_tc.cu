@@ -408,6 +408,9 @@ void ts_tc_set_fault(ts_plan p, int stall_copies, unsigned wait_limit) {
   t.stall_copies = stall_copies;
   t.wait_limit = wait_limit;
 }
+bool ts_tc_stalled(ts_plan p) {
+  return p->tc && static_cast<ts_tc_tables *>(p->tc)->tab.stall_copies;
+}
 const int *ts_tc_w_kmin(ts_plan p) {
   const auto *t = static_cast<ts_tc_tables *>(p->tc);
   return t ? t->w_kmin : nullptr;
@@ -660,6 +663,13 @@ void ts_launch_leg_analys_tc(ts_plan p, const float2 *g, long gs, float2 *out, l
 // allows it, else spat -> G scratch -> w image; then -> q
 void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf, cudaStream_t s) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
+  if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s)) {
+    const long field = (long)(p->mmax + 1) * p->nlat;
+    t->gscratch.ensure(sizeof(float2) * field * nf);
+    ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
+    ts_launch_leg_analys_gemm(p, (const float2 *)t->gscratch.p, field, (float2 *)qlm, p->nlm, nf, s);
+    return;
+  }
   ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS));
   if (!ts_launch_fourier_analys_w(p, spat, ss, nf, TS_TC_FIELDS, (char *)t->wimg.p, s)) {
     const long field = (long)(p->mmax + 1) * p->nlat;
