@@ -619,9 +619,13 @@ constexpr long ts_f2_smem_bytes(int nb) {
 // Resident CTAs per SM asked of the register allocator.  Transform kernels
 // with P <= 24: 1152 threads per SM (<= 56 registers each), else whatever
 // fits.  The fused phase keeps every species' P grid points of a row in
-// registers (~170 registers): no limit.
+// registers: with one or two species, CTAs of at most 256 threads are held to
+// 128 registers (they would take 142), so that two share an SM; larger CTAs
+// and more species get what they need (168 at P = 24, where two CTAs would
+// spill).  The phase of 256 Brusselator instances at lmax 127 (P = 16): one CTA
+// an SM 150 us, two 110 us.
 #define TS_F2_MINB(P, R) ((P) <= 24 ? 1152 / ((P) * (R)) : 1)
-#define TS_F2_PHASE_MINB(P, R) 1
+#define TS_F2_PHASE_MINB(NB, P, R) ((NB) <= 2 && (P) * (R) <= 256 ? 2 : 1)
 
 // fm[field][m][lat] -> spat[field][lat][phi].  grid = (ceil(nlat/R), fields),
 // block = P*R.  Rows leave by bulk copies when the field's grid is 16-byte
@@ -830,7 +834,7 @@ TS_DEV void ts_f2_groups(F &&f) {
 // pair of barriers and one batch of loads per pair (the registers of two
 // P-point rows per thread are what the middle section holds anyway).
 template <class Prog, int P, int Q, int R, bool PAIRED>
-__global__ void __launch_bounds__(P *R, TS_F2_PHASE_MINB(P, R))
+__global__ void __launch_bounds__(P *R, TS_F2_PHASE_MINB(Prog::NSYN > Prog::NANA ? Prog::NSYN : Prog::NANA, P, R))
 ts_f2_phase(TsFftTab ft, TsPhaseIO io) {
   using C = TsF2<P, Q, R>;
   constexpr int NSYN = Prog::NSYN, NGIN = Prog::NGIN, NANA = Prog::NANA, NGOUT = Prog::NGOUT;
