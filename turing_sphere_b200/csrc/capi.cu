@@ -119,6 +119,12 @@ void ts_analys_dev(ts_plan p, const float *spat, float *qlm, int batch, cudaStre
   ts_launch_leg_analys(p, fm, fm_stride, (float2 *)qlm, p->nlm, batch, s);
 }
 
+std::vector<const void *> ts_plan_scratch(ts_plan p) {
+  std::vector<const void *> v{p->fm.p, p->adj_grid.p, p->adj_spec.p, p->lg_tab};
+  ts_tc_scratch(p, &v);
+  return v;
+}
+
 namespace {
 void synth_dev(ts_plan p, const float *qlm, float *spat, int batch, cudaStream_t s) {
   ts_synth_dev(p, qlm, spat, batch, s);

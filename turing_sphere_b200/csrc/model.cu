@@ -184,6 +184,16 @@ struct Adjoint {
   double *pbar = nullptr;         // [instance][nparams]
   float *tmp = nullptr;           // transform-adjoint output
   std::vector<float *> owned;
+  // forward_backward's own memory: checkpoints, a segment's states, cotangents
+  // [state] and the states a tape starts from, kept from call to call
+  ts_dbuf ck, seg, lam, cur;
+  // one replayed step (tape, its final states to `cur`) and one reverse step
+  // (tape, adjoint) as graphs; they hold pointers into the plan's scratch, so
+  // they are dropped when that has moved since the capture
+  cudaGraphExec_t fwd_graph = nullptr, rev_graph = nullptr;
+  std::vector<const void *> key;
+  int eager_left = 4;  // steps of each kind run eagerly first (scratch then has its size)
+  bool graphs_ok = true;
 };
 
 struct ts_model_s {
@@ -1177,7 +1187,16 @@ void adj_prepare(ts_model m) {
   A.ready = true;
 }
 
+void adj_drop_graphs(Adjoint &A) {
+  for (cudaGraphExec_t *g : {&A.fwd_graph, &A.rev_graph}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
 void adj_free(Adjoint &A) {
+  adj_drop_graphs(A);
+  for (ts_dbuf *b : {&A.ck, &A.seg, &A.lam, &A.cur}) b->release();
   for (float *q : A.owned) cudaFree(q);
   A.owned.clear();
   if (A.pbar) cudaFree(A.pbar);
@@ -1288,6 +1307,57 @@ void adj_reverse(ts_model m, const std::vector<float *> &lam, cudaStream_t st) {
                             cudaMemcpyDeviceToDevice, st));
 }
 
+// What a replayed or reverse step's graph was captured with, beside memory
+// that belongs to the model and does not move.
+std::vector<const void *> adj_key(ts_model m) {
+  std::vector<const void *> k = ts_plan_scratch(m->plan);
+  k.push_back(m->adj.lam.p);
+  k.push_back(m->adj.cur.p);
+  return k;
+}
+
+// `run` (only launches, copies and memsets on `st`) by way of the graph in
+// *exec, captured on first use; eagerly when graphs are off, cannot be used on
+// this stream or fail to capture, and for the first steps
+template <class F>
+void adj_graphed(ts_model m, cudaGraphExec_t *exec, cudaStream_t st, F &&run) {
+  Adjoint &A = m->adj;
+  if (A.eager_left > 0 || !A.graphs_ok || !graphs_usable(m)) {
+    if (A.eager_left > 0) A.eager_left--;
+    run();
+    return;
+  }
+  const std::vector<const void *> key = adj_key(m);
+  if (key != A.key) {
+    adj_drop_graphs(A);
+    A.key = key;
+  }
+  if (!*exec) {
+    cudaGraph_t graph = nullptr;
+    bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (ok) {
+      try {
+        run();
+      } catch (const ts_exc &) {
+        ok = false;
+      }
+      const bool ended = cudaStreamEndCapture(st, &graph) == cudaSuccess;
+      ok = ok && ended && graph && adj_key(m) == key;
+    }
+    if (ok) ok = cudaGraphInstantiate(exec, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
+    if (!ok) {
+      (void)cudaGetLastError();
+      *exec = nullptr;
+      A.graphs_ok = false;
+      adj_drop_graphs(A);
+      run();
+      return;
+    }
+  }
+  TS_CUDA(cudaGraphLaunch(*exec, st));
+}
+
 void free_model(ts_model m) {
   adj_free(m->adj);
   drop_graphs(m);
@@ -1306,17 +1376,6 @@ void free_model(ts_model m) {
   m->wimg.release();
   if (m->lib) cudaLibraryUnload(m->lib);
 }
-
-// device memory released at scope exit
-struct DevMem {
-  void *p = nullptr;
-  explicit DevMem(size_t bytes) { TS_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16))); }
-  ~DevMem() {
-    if (p) cudaFree(p);
-  }
-  DevMem(const DevMem &) = delete;
-  DevMem &operator=(const DevMem &) = delete;
-};
 
 float *dalloc(long n) {
   float *p = nullptr;
@@ -1772,10 +1831,14 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   const int B = m->batch, ns = (int)m->state.size();
   const long sz = 2 * m->plan->nlm * (long)B;  // floats of one state, all instances
   const int nseg = (nsteps + every - 1) / every;
-  // checkpoints [segment][state], segment states [step][state], cotangents [state]
-  DevMem ck(sizeof(float) * sz * ns * nseg), seg(sizeof(float) * sz * ns * every),
-      lamb(sizeof(float) * sz * ns);
-  float *pck = (float *)ck.p, *pseg = (float *)seg.p, *plam = (float *)lamb.p;
+  // checkpoints [segment][state], segment states [step][state], cotangents
+  // [state], and the states [state] a tape starts from
+  A.ck.ensure(sizeof(float) * sz * ns * nseg);
+  A.seg.ensure(sizeof(float) * sz * ns * every);
+  A.lam.ensure(sizeof(float) * sz * ns);
+  A.cur.ensure(sizeof(float) * sz * ns);
+  float *pck = (float *)A.ck.p, *pseg = (float *)A.seg.p, *plam = (float *)A.lam.p,
+        *pcur = (float *)A.cur.p;
   for (int i = 0; i < nsteps; i += every) {
     for (int s = 0; s < ns; s++)
       TS_CUDA(cudaMemcpyAsync(pck + ((long)(i / every) * ns + s) * sz, m->host.at(m->state[s]).cur,
@@ -1785,25 +1848,33 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   TS_CUDA(cudaMemcpyAsync(plam, final_bar, sizeof(float) * sz * ns, cudaMemcpyHostToDevice, st));
   TS_CUDA(cudaMemsetAsync(A.pbar, 0, sizeof(double) * std::max<size_t>(m->params.size(), 1) * B, st));
   std::vector<float *> lam(ns);
-  for (int s = 0; s < ns; s++) lam[s] = plam + (long)s * sz;
+  std::vector<const float *> cur(ns);
+  for (int s = 0; s < ns; s++) {
+    lam[s] = plam + (long)s * sz;
+    cur[s] = pcur + (long)s * sz;
+  }
+  auto copy = [&](float *dst, const float *src) {
+    TS_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * sz * ns, cudaMemcpyDeviceToDevice, st));
+  };
   for (int g = nseg - 1; g >= 0; g--) {
     const int len = std::min(every, nsteps - g * every);
-    TS_CUDA(cudaMemcpyAsync(pseg, pck + (long)g * ns * sz, sizeof(float) * sz * ns,
-                            cudaMemcpyDeviceToDevice, st));
-    auto states = [&](int j) {
-      std::vector<const float *> v(ns);
-      for (int s = 0; s < ns; s++) v[s] = pseg + ((long)j * ns + s) * sz;
-      return v;
-    };
+    copy(pcur, pck + (long)g * ns * sz);
+    copy(pseg, pcur);
     for (int j = 1; j < len; j++) {  // replay the segment: the state before every step
-      adj_tape(m, states(j - 1), st);
-      for (int s = 0; s < ns; s++)
-        TS_CUDA(cudaMemcpyAsync(pseg + ((long)j * ns + s) * sz, A.val[A.state_out[s]],
-                                sizeof(float) * sz, cudaMemcpyDeviceToDevice, st));
+      adj_graphed(m, &A.fwd_graph, st, [&] {
+        adj_tape(m, cur, st);
+        for (int s = 0; s < ns; s++)
+          TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
+                                  cudaMemcpyDeviceToDevice, st));
+      });
+      copy(pseg + (long)j * ns * sz, pcur);
     }
     for (int j = len - 1; j >= 0; j--) {
-      adj_tape(m, states(j), st);
-      adj_reverse(m, lam, st);
+      if (j < len - 1) copy(pcur, pseg + (long)j * ns * sz);
+      adj_graphed(m, &A.rev_graph, st, [&] {
+        adj_tape(m, cur, st);
+        adj_reverse(m, lam, st);
+      });
     }
   }
   TS_CUDA(cudaMemcpyAsync(init_bar, plam, sizeof(float) * sz * ns, cudaMemcpyDeviceToHost, st));
@@ -1812,6 +1883,16 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
                             cudaMemcpyDeviceToHost, st));
   TS_CUDA(cudaStreamSynchronize(st));
   TS_CUDA(cudaGetLastError());
+  // small workspaces stay for the next call, large ones go back
+  if (A.ck.cap + A.seg.cap > (size_t)256 << 20) {
+    A.ck.release();
+    A.seg.release();
+  }
+  if (A.lam.cap + A.cur.cap > (size_t)256 << 20) {
+    adj_drop_graphs(A);
+    A.lam.release();
+    A.cur.release();
+  }
   TSM_END
 }
 
@@ -1819,6 +1900,7 @@ int ts_model_set_graphs(ts_model m, int enable) {
   TSM_BEGIN(m)
   m->use_graphs = enable != 0;
   drop_graphs(m);
+  adj_drop_graphs(m->adj);
   TSM_END
 }
 

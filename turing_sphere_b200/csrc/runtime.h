@@ -131,6 +131,10 @@ void ts_analys_dev(ts_plan p, const float *spat, float *qlm, int batch, cudaStre
 void ts_synth_adjoint(ts_plan p, const float *gbar, float *qbar, int nf, cudaStream_t s);
 void ts_analys_adjoint(ts_plan p, const float *qbar, float *gbar, int nf, cudaStream_t s);
 
+// the plan's scratch buffers as they are now: a captured graph that holds their
+// addresses is good as long as none has moved
+std::vector<const void *> ts_plan_scratch(ts_plan p);
+
 // autotune.cu: time the candidate kernel shapes of a plan, keep the fastest
 void ts_autotune(ts_plan p);
 // rows per two-phase FFT CTA in use (0 when the plan's rows have no shape)
@@ -209,6 +213,7 @@ struct TsTcGeom {
 TsTcGeom ts_tc_geom(ts_plan p);
 void ts_tc_set_fault(ts_plan p, int stall_copies, unsigned wait_limit);
 bool ts_tc_stalled(ts_plan p);
+void ts_tc_scratch(ts_plan p, std::vector<const void *> *out);
 // tiles / chunks the tensor-core polar skip drops
 void ts_tc_skip_counts(ts_plan p, int *tiles, int *chunks);
 // per (32-latitude chunk, parity): the order m from which the W image's chunk

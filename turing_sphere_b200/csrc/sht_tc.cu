@@ -411,6 +411,14 @@ void ts_tc_set_fault(ts_plan p, int stall_copies, unsigned wait_limit) {
 bool ts_tc_stalled(ts_plan p) {
   return p->tc && static_cast<ts_tc_tables *>(p->tc)->tab.stall_copies;
 }
+void ts_tc_scratch(ts_plan p, std::vector<const void *> *out) {
+  const auto *t = static_cast<ts_tc_tables *>(p->tc);
+  if (!t) return;
+  for (const void *q : {t->qimg.p, t->wimg.p, t->gscratch.p, (void *)t->synth, (void *)t->anal})
+    out->push_back(q);
+  // the test hook's settings travel as kernel arguments
+  out->push_back(reinterpret_cast<const void *>((uintptr_t)t->tab.stall_copies << 32 | t->tab.wait_limit));
+}
 const int *ts_tc_w_kmin(ts_plan p) {
   const auto *t = static_cast<ts_tc_tables *>(p->tc);
   return t ? t->w_kmin : nullptr;
