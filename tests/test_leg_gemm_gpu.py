@@ -144,3 +144,28 @@ def test_batches_of_a_tensor_core_plan(device, parity, lmax, mmax, nlat, nphi, b
     parity(f"tf32x3 lmax{lmax} mmax{mmax} nlat{nlat} B{batch} synth", worst[0], TOL)
     parity(f"tf32x3 lmax{lmax} mmax{mmax} nlat{nlat} B{batch} analys", worst[1], TOL)
     plan.destroy()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("lmax,mmax,nlat,nphi", [(63, 63, 96, 192), (64, 60, 131, 256), (97, 97, 100, 256),
+                                                 (130, 130, 263, 768), (255, 255, 384, 768)])
+def test_one_and_two_fields(device, parity, precision, lmax, mmax, nlat, nphi):
+    """The kernels without staging: rows of 16, 32 and 64 degrees, one and two
+    CTAs to an order, odd latitudes; both fields against the oracle."""
+    import torch
+    plan = ShtPlan.create(device, ShtConfig(lmax, mmax, nlat, nphi), {"precision": precision})
+    ref = O.ShtReference(lmax, mmax, nlat, nphi)
+    q = np.stack([spectrum(lmax, mmax, 5 + k) for k in range(2)])
+    want = np.stack([ref.synth(x.astype(np.float64)) for x in q])
+    g = want.astype(np.float32)
+    back = np.stack([ref.analys(x.astype(np.float64)) for x in g])
+    for batch in (1, 2):
+        for name, call, x, y in (("synth", plan.synth_dev, q, want), ("analys", plan.analys_dev, g, back)):
+            src = torch.from_numpy(x[2 - batch:]).cuda()
+            dst = torch.full((batch, y.shape[1]), float("nan"), device="cuda")
+            torch.cuda.synchronize()
+            call(src.data_ptr(), dst.data_ptr(), batch)
+            device.sync()
+            worst = max(O.rel_l2(dst[f].cpu().numpy(), y[2 - batch + f]) for f in range(batch))
+            parity(f"{precision} lmax{lmax} mmax{mmax} nlat{nlat} B{batch} {name}", worst, TOL)
+    plan.destroy()

@@ -281,14 +281,14 @@ struct TsLg {
   static constexpr int NF = NCOL / 2;        // fields
   static constexpr int A = 2 * TS_LG_KT * TS_LG_ROWS;  // floats of a stage's table values
   // synthesis: a stage's coefficients [field][2 KT degrees] (an odd pitch in
-  // complex values: the lanes' fields fall in distinct banks), 2 stages
+  // complex values: the lanes' fields fall in distinct banks)
   static constexpr int QP = 2 * TS_LG_KT + 1;
   static constexpr int SB = 2 * QP * NF;
   static constexpr int SP = 2 * TS_LG_ROWS + 4;  // staging: floats per (parity, field)
   static constexpr int SYN = 2 * (A + SB), SSTG = 2 * NF * SP;
   static constexpr int SYN_SMEM = sizeof(float) * (SYN > SSTG ? SYN : SSTG);
-  // analysis: a stage's columns [parity][latitude][field re, im], 2 stages,
-  // and the grid values they are folded from, NR pairs per thread
+  // analysis: the grid values of a stage, NR pairs per thread, and the columns
+  // [parity][latitude][field re, im] folded from them, 2 stages
   static constexpr int BP = NCOL + 4;
   static constexpr int AB = 2 * TS_LG_KT * BP;
   static constexpr int NR = NF / 8;
@@ -637,5 +637,191 @@ ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, lo
       }
       epi(f0 / Epi::NA + q, lm0 + i, v);
     }
+  }
+}
+
+// ------------------------------------------------------------- few fields
+//
+// One or two fields: every table value meets two or four numbers, so the
+// products are bound by reading the table (25 MB a direction at lmax 255, from
+// the L2) and by the latency of a CTA's few stages.  No staging then: a warp's lanes read whole rows of the table
+// straight into registers, pairs of neighbours each, with eight rows in flight,
+// and the columns come as broadcasts from shared memory.  The rows of a CTA are
+// dealt out to its warps, whose sums are added up at the end.
+
+template <int F>
+TS_DEV void ts_lg_columns(float2 (&c)[F], const float2 *s) {
+  if constexpr (F == 1) {
+    c[0] = s[0];
+  } else {
+#pragma unroll
+    for (int f = 0; f < F; f += 2) {
+      const float4 x = *reinterpret_cast<const float4 *>(s + f);
+      c[f] = make_float2(x.x, x.y);
+      c[f + 1] = make_float2(x.z, x.w);
+    }
+  }
+}
+
+// grid = (nhp / 64, mmax + 1), 256 threads: warp = (parity, one of 4 parts of
+// its degrees), lane = 2 of 64 latitudes.  Shared memory: (lmax + 1) F float2.
+template <int F>
+__global__ void __launch_bounds__(256)
+ts_leg_synth_few(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ fm, long fm_stride,
+                 int nfields) {
+  extern __shared__ __align__(16) float2 ts_smem_fs[];
+  __shared__ float2 red[8][F][TS_LG_ROWS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, par = warp & 1, part = warp >> 1;
+  const int lat0 = blockIdx.x * TS_LG_ROWS, m = blockIdx.y, K = t.lmax - m + 1;
+  const long base = ts_lm_base(t.lmax, m);
+  const int *on = g.onset + (long)m * g.nhp + lat0 + 2 * lane;
+  const int o0 = __ldg(on), o1 = __ldg(on + 1);
+  const float2 *src[F];
+#pragma unroll
+  for (int f = 0; f < F; f++) src[f] = ts_field(q, min(f, nfields - 1)) + base;
+  for (int i0 = tid; i0 < K; i0 += 1024) {  // every load of a thread before its stores
+    float2 v[4][F];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int f = 0; f < F; f++) v[u][f] = __ldg(src[f] + min(i0 + 256 * u, K - 1));
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int f = 0; f < F; f++)
+        if (i0 + 256 * u < K) ts_smem_fs[(i0 + 256 * u) * F + f] = v[u][f];
+  }
+  const int first = __reduce_min_sync(0xffffffffu, min(o0, o1));
+  const int kp = ts_lg_kpar(t.lmax, m, par);
+  const float *row = g.tab + (ts_lg_off(t.lmax, m) + (par ? ts_lg_k16(t.lmax, m, 0) : 0)) * g.nhp + lat0 + 2 * lane;
+  float2 acc[F][2];
+#pragma unroll
+  for (int f = 0; f < F; f++) acc[f][0] = acc[f][1] = make_float2(0.f, 0.f);
+  __syncthreads();
+  for (int j = (first >> 1) + part; j < kp; j += 32) {
+    float2 p[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      p[u] = j + 4 * u < kp ? __ldg(reinterpret_cast<const float2 *>(row + (long)(j + 4 * u) * g.nhp))
+                            : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      float2 c[F];
+      ts_lg_columns<F>(c, ts_smem_fs + (2 * min(j + 4 * u, kp - 1) + par) * F);
+#pragma unroll
+      for (int f = 0; f < F; f++) {
+        ts_fma2(acc[f][0], make_float2(p[u].x, p[u].x), c[f]);
+        ts_fma2(acc[f][1], make_float2(p[u].y, p[u].y), c[f]);
+      }
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < F; f++) {
+    red[warp][f][2 * lane] = acc[f][0];
+    red[warp][f][2 * lane + 1] = acc[f][1];
+  }
+  __syncthreads();
+  for (int i = tid; i < TS_LG_ROWS * F; i += 256) {
+    const int f = i / TS_LG_ROWS, r = i % TS_LG_ROWS, lat = lat0 + r, south = t.nlat - 1 - lat;
+    if (f >= nfields || lat >= t.nh) continue;
+    float2 e = red[0][f][r], o = red[1][f][r];
+#pragma unroll
+    for (int k = 2; k < 8; k += 2) {
+      e = c_add(e, red[k][f][r]);
+      o = c_add(o, red[k + 1][f][r]);
+    }
+    float2 *dst = fm + (long)f * fm_stride + (long)m * t.nlat;
+    dst[lat] = c_add(e, o);
+    if (south != lat) dst[south] = c_sub(e, o);
+  }
+}
+
+// grid = (ceil((lmax + 1) / 128), mmax + 1), 512 threads: 64 degrees of each
+// parity per CTA; warp = (parity, one of 8 parts of the latitudes), lane = 2
+// degrees (rows of up to 16 or 32 degrees: 4 or 2 latitudes a load).  Shared
+// memory: 2 nh F + 16 F 64 float2.
+template <int F, class Epi>
+__global__ void __launch_bounds__(512)
+ts_leg_analys_few(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, long g_stride, Epi epi,
+                  int nfields) {
+  extern __shared__ __align__(16) float2 ts_smem_fa[];  // [parity][latitude][F], then [warp][F][64]
+  __shared__ int first;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, par = warp & 1, part = warp >> 1;
+  const int m = blockIdx.y, j0 = blockIdx.x * TS_LG_ROWS, K = t.lmax - m + 1;
+  if (2 * j0 >= K) return;
+  const int kp0 = ts_lg_k16(t.lmax, m, 0), kp = par ? ts_lg_k16(t.lmax, m, 1) : kp0;
+  if (tid == 0) first = t.nh;
+  __syncthreads();
+  for (int lat = tid; lat < t.nh; lat += 512) {
+    if (__ldg(g.onset + (long)m * g.nhp + lat) < 2 * (j0 + TS_LG_ROWS)) atomicMin(&first, lat);
+    const int south = t.nlat - 1 - lat;
+    const float w = __ldg(t.wq + lat);
+#pragma unroll
+    for (int f = 0; f < F; f++) {
+      float2 n = make_float2(0.f, 0.f), s = n;
+      if (f < nfields) {
+        const float2 *src = gm + (long)f * g_stride + (long)m * t.nlat;
+        n = __ldg(src + lat);
+        if (south != lat) s = __ldg(src + south);
+      }
+      ts_smem_fa[lat * F + f] = c_scale(c_add(n, s), w);
+      ts_smem_fa[(t.nh + lat) * F + f] = c_scale(c_sub(n, s), w);
+    }
+  }
+  __syncthreads();
+  const int jn = min(TS_LG_ROWS, kp - j0);  // (a multiple of 16, or none)
+  const int lpr = jn <= 16 ? 8 : jn <= 32 ? 16 : 32, rpw = 32 / lpr;  // lanes of a row, rows of a load
+  const int sub = lane / lpr, jl = 2 * (lane & (lpr - 1));
+  const bool on = jl < jn;
+  const float *row = g.tab + ts_lg_off(t.lmax, m) * g.nhp + (par ? (long)kp0 * g.nhp : 0) + j0 + (on ? jl : 0);
+  const float2 *col = ts_smem_fa + par * t.nh * F;
+  float2 acc[F][2];
+#pragma unroll
+  for (int f = 0; f < F; f++) acc[f][0] = acc[f][1] = make_float2(0.f, 0.f);
+  const int step = 8 * rpw;
+  if (on)
+    for (int lat = first + part * rpw + sub; lat < t.nh; lat += 8 * step) {
+      float2 p[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        p[u] = lat + u * step < t.nh ? __ldg(reinterpret_cast<const float2 *>(row + (long)(lat + u * step) * kp))
+                                     : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        float2 c[F];
+        ts_lg_columns<F>(c, col + min(lat + u * step, t.nh - 1) * F);
+#pragma unroll
+        for (int f = 0; f < F; f++) {
+          ts_fma2(acc[f][0], make_float2(p[u].x, p[u].x), c[f]);
+          ts_fma2(acc[f][1], make_float2(p[u].y, p[u].y), c[f]);
+        }
+      }
+    }
+  float2 *red = ts_smem_fa + 2 * t.nh * F;
+#pragma unroll
+  for (int f = 0; f < F; f++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      float2 v = acc[f][e];
+      for (int d = lpr; d < 32; d <<= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, d);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, d);
+      }
+      if (on && sub == 0) red[(warp * F + f) * TS_LG_ROWS + jl + e] = v;
+    }
+  __syncthreads();
+  const long lm0 = ts_lm_base(t.lmax, m) + 2 * j0;
+  const int n = min(2 * TS_LG_ROWS, K - 2 * j0), ni = nfields / Epi::NA;
+  for (int i = tid; i < n * ni; i += 512) {
+    const int inst = i / n, d = i % n;
+    float2 v[Epi::NA];
+#pragma unroll
+    for (int a = 0; a < Epi::NA; a++) {
+      const float2 *r = red + ((d & 1) * F + inst * Epi::NA + a) * TS_LG_ROWS + (d >> 1);
+      v[a] = r[0];
+#pragma unroll
+      for (int k = 1; k < 8; k++) v[a] = c_add(v[a], r[2 * k * F * TS_LG_ROWS]);
+    }
+    epi(inst, lm0 + d, v);
   }
 }

@@ -75,6 +75,31 @@ void analys_t(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, const
   kernel<<<grid, TS_LG_THREADS, S::ANA_SMEM, s>>>(p->leg, g, gm, gs, out, nf, S::NF);
 }
 
+template <int F>
+void synth_few(ts_plan p, const TsLegGemmTab &g, const TsFields &q, float2 *fm, long fs, int nf,
+               cudaStream_t s) {
+  const size_t smem = sizeof(float2) * (size_t)(p->lmax + 1) * F;
+  ts_allow_smem((const void *)ts_leg_synth_few<F>, p->ctx->device, smem);
+  ts_leg_synth_few<F><<<dim3(g.nhp / TS_LG_ROWS, p->mmax + 1), 256, smem, s>>>(p->leg, g, q, fm, fs, nf);
+}
+
+size_t few_smem(ts_plan p, int F) { return sizeof(float2) * F * (2 * (size_t)p->nh + 16 * TS_LG_ROWS); }
+
+template <int F>
+void analys_few(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, const TsLgStore &out,
+                int nf, cudaStream_t s) {
+  const auto kernel = ts_leg_analys_few<F, TsLgStore>;
+  ts_allow_smem((const void *)kernel, p->ctx->device, few_smem(p, F));
+  dim3 grid((p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS), p->mmax + 1);
+  kernel<<<grid, 512, few_smem(p, F), s>>>(p->leg, g, gm, gs, out, nf);
+}
+
+// One or two fields take the kernels without staging (us, tiled | these, lmax
+// 255: synthesis 1 field 12.5 | 9.2, 2: 12.6 | 10.5, 4: 12.5 | 12.7; analysis 1:
+// 16.8 | 10.4, 2: 16.8 | 10.5, 4: 17.4 | 14.7; lmax 1023, whole transforms:
+// synthesis 1: 343 | 222, 4: 389 | 426; analysis 1: 382 | 252, 4: 425 | 486).
+bool lg_few(int nf) { return nf <= 2; }
+
 }  // namespace
 
 // Which calls take the products.  On B200 (us, recurrence kernel | product):
@@ -146,7 +171,9 @@ bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fs,
                               cudaStream_t s) {
   if (!ts_lg_use(p, nf, false) || !lg_ready(p, s)) return false;
   const TsLegGemmTab &g = p->lg_syn;
-  switch (lg_ncol(nf, 1)) {
+  if (lg_few(nf))
+    nf == 1 ? synth_few<1>(p, g, q, fm, fs, nf, s) : synth_few<2>(p, g, q, fm, fs, nf, s);
+  else switch (lg_ncol(nf, 1)) {
     case 64: synth_t<64>(p, g, q, fm, fs, nf, s); break;
     case 32: synth_t<32>(p, g, q, fm, fs, nf, s); break;
     default: synth_t<16>(p, g, q, fm, fs, nf, s); break;
@@ -163,7 +190,9 @@ bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *gm, long gs, float2 *out
   st.base[0] = out;
   st.inst_stride[0] = os;
   st.nper = 1;
-  switch (lg_ncol(nf, 1)) {
+  if (lg_few(nf))
+    nf == 1 ? analys_few<1>(p, g, gm, gs, st, nf, s) : analys_few<2>(p, g, gm, gs, st, nf, s);
+  else switch (lg_ncol(nf, 1)) {
     case 64: analys_t<64>(p, g, gm, gs, st, nf, s); break;
     case 32: analys_t<32>(p, g, gm, gs, st, nf, s); break;
     default: analys_t<16>(p, g, gm, gs, st, nf, s); break;
@@ -175,11 +204,22 @@ bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *gm, long gs, float2 *out
 bool ts_lg_prepare(ts_plan p, cudaStream_t s) { return lg_ready(p, s); }
 
 void ts_lg_analys_shape(ts_plan p, int nf, int na, TsLgShape *sh) {
+  const unsigned chunks = (p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS), M = p->mmax + 1;
+  if (lg_few(nf)) {
+    sh->few = nf;
+    sh->per_cta = nf;
+    sh->threads = 512;
+    sh->smem = few_smem(p, nf);
+    sh->grid[0] = chunks;
+    sh->grid[1] = M;
+    sh->grid[2] = 1;
+    return;
+  }
   sh->ncol = lg_ncol(nf, na);
   sh->per_cta = na * (sh->ncol / 2 / na);
   sh->threads = TS_LG_THREADS;
   sh->smem = sh->ncol == 64 ? TsLg<64>::ANA_SMEM : sh->ncol == 32 ? TsLg<32>::ANA_SMEM : TsLg<16>::ANA_SMEM;
-  sh->grid[0] = (p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS);
+  sh->grid[0] = chunks;
   sh->grid[1] = (nf + sh->per_cta - 1) / sh->per_cta;
-  sh->grid[2] = p->mmax + 1;
+  sh->grid[2] = M;
 }

@@ -59,7 +59,7 @@ struct Stage {
   int lb = 0, F = 1, K = 1, W = 1, per_cta = 1;
   int threads = 0;    // phase: threads per CTA (two-phase FFT: P*R, lb = R rows)
   bool wimg = false;  // tensor-core plan: the phase writes the W image itself
-  TsLgShape lg{};     // LegAnalys of a batch on an FP32 plan: the products' shape (ncol 0: recurrence)
+  TsLgShape lg{};     // LegAnalys of a batch on an FP32 plan: the products' shape (threads 0: recurrence)
   size_t smem = 0;
   // SpecEW: the variant that takes four consecutive coefficients per thread
   // (float4 loads and stores; used when every array and stride allows it)
@@ -592,7 +592,7 @@ void schedule(ts_model m, Program &P, bool is_step) {
         ts_analys_shape(p, m->batch * st.nana, st.nana, &st.F, &st.K, &st.W, &st.per_cta);
       }
     }
-    if (st.lg.ncol) {
+    if (st.lg.threads) {
       // epilogue of the products: one instance's NA analysed values of one
       // coefficient, re and im, with the state read and written as pairs
       Emitter ev{f, {}};
@@ -634,7 +634,8 @@ void schedule(ts_model m, Program &P, bool is_step) {
         src << "    *reinterpret_cast<float2 *>(io.sout[" << o << "] + inst * io.sout_stride[" << o
             << "] + 2 * lm) = make_float2(ro[" << o << "], io_[" << o << "]);\n";
       src << "  }\n};\n";
-      st.expr = "ts_leg_analys_gemm<" + std::to_string(st.lg.ncol) + ", " + en + ">";
+      st.expr = st.lg.few ? "ts_leg_analys_few<" + std::to_string(st.lg.few) + ", " + en + ">"
+                          : "ts_leg_analys_gemm<" + std::to_string(st.lg.ncol) + ", " + en + ">";
       st.label = "legana  " + std::to_string(na) + " field(s), " + std::to_string(E.size()) +
                  " spectral statement(s) fused";
       st.src = src.str();
@@ -882,9 +883,9 @@ void run_program(ts_model m, Program &P, cudaStream_t st) {
         long gs = field;
         int nfields = B * s.nana;
         int per_cta = s.per_cta;
-        if (s.lg.ncol) {
+        if (s.lg.threads) {
           TsLegGemmTab tab = p->lg_ana;
-          void *args[] = {&leg, &tab, &g, &gs, &epi, &nfields, &per_cta};
+          void *args[] = {&leg, &tab, &g, &gs, &epi, &nfields, &per_cta};  // (few: without per_cta)
           TS_CUDA(cudaLaunchKernel((const void *)s.kern, dim3(s.lg.grid[0], s.lg.grid[1], s.lg.grid[2]),
                                    dim3(s.lg.threads), args, s.smem, st));
         } else if (p->precision != TS_PREC_FP32) {
@@ -944,7 +945,7 @@ void finish_shapes(ts_model m) {
         const int nrows = s.nsyn + s.nana + 1;
         if (!s.threads) s.lb = ts_fourier_lb(p, m->batch, nrows, &s.smem);
       } else if (s.kind == Stage::LegAnalys) {
-        s.smem = s.lg.ncol ? s.lg.smem
+        s.smem = s.lg.threads ? s.lg.smem
                  : p->precision != TS_PREC_FP32 ? ts_tc_analys_smem(p) : ts_analys_smem(p, s.F, s.W);
       }
     }
@@ -1527,7 +1528,7 @@ int ts_model_compile(ts_plan plan, const char *source, const char *const *state,
       size_t wb = 0;
       for (auto &P : m->prog)
         for (auto &st : P.stages)
-          if (st.kind == Stage::LegAnalys && !st.lg.ncol)
+          if (st.kind == Stage::LegAnalys && !st.lg.threads)
             wb = std::max(wb, ts_tc_wimg_bytes(plan, batch * st.nana, st.per_cta));
       m->wimg.ensure(std::max<size_t>(wb, 16));
       TS_CUDA(cudaMemset(m->wimg.p, 0, m->wimg.cap));

@@ -168,9 +168,10 @@ bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fm_
                               int nfields, cudaStream_t s);
 bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *g, long g_stride, float2 *q, long q_stride,
                                int nfields, cudaStream_t s);
-// launch shape of the analysis of nf fields in whole instances of na
+// launch shape of the analysis of nf fields in whole instances of na:
+// ts_leg_analys_few<few, Epi>, or ts_leg_analys_gemm<ncol, Epi>
 struct TsLgShape {
-  int ncol, per_cta, threads;
+  int few, ncol, per_cta, threads;
   size_t smem;
   unsigned grid[3];
 };
