@@ -617,21 +617,26 @@ constexpr long ts_f2_smem_bytes(int nb) {
 // ---------------------------------------------------------------- kernels
 
 // Resident CTAs per SM asked of the register allocator.  Transform kernels
-// with P <= 24: 1152 threads per SM (<= 56 registers each), else whatever
-// fits.  The fused phase keeps every species' P grid points of a row in
-// registers: with one or two species, CTAs of at most 256 threads are held to
-// 128 registers (they would take 142), so that two share an SM; larger CTAs
-// and more species get what they need (168 at P = 24, where two CTAs would
-// spill).  The phase of 256 Brusselator instances at lmax 127 (P = 16): one CTA
-// an SM 150 us, two 110 us.
-#define TS_F2_MINB(P, R) ((P) <= 24 ? 1152 / ((P) * (R)) : 1)
+// with P <= 24: 1152 threads per SM (<= 56 registers each).  P = 32 on 8 rows:
+// three CTAs of 256 threads (80 registers, no spills; they would take 100) or,
+// at Q = 32, the two that shared memory holds; its 16-row form keeps one CTA of
+// 512, P = 48 one of 384 (two would spill: 201 -> 225 us at nphi 3072).  64
+// fields at lmax 511 (nphi 1536): synthesis 178 us with 16 rows, 159 with 8 and
+// two CTAs, 141 with three.  The fused phase keeps every species' P grid points
+// of a row in registers: with one or two species, CTAs of at most 256 threads
+// are held to 128 registers (they would take 142), so that two share an SM;
+// larger CTAs and more species get what they need (168 at P = 24, where two
+// CTAs would spill).  The phase of 256 Brusselator instances at lmax 127
+// (P = 16): one CTA an SM 150 us, two 110 us.
+#define TS_F2_MINB(P, Q, R) \
+  ((P) <= 24 ? 1152 / ((P) * (R)) : (P) == 32 && (R) == 8 ? ((Q) <= 24 ? 3 : 2) : 1)
 #define TS_F2_PHASE_MINB(NB, P, R) ((NB) <= 2 && (P) * (R) <= 256 ? 2 : 1)
 
 // fm[field][m][lat] -> spat[field][lat][phi].  grid = (ceil(nlat/R), fields),
 // block = P*R.  Rows leave by bulk copies when the field's grid is 16-byte
 // aligned (fewer, larger memory instructions), else by per-thread stores.
 template <int P, int Q, int R>
-__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, R))
+__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
 ts_f2_synth(TsFftTab ft, const float2 *__restrict__ fm, long fm_stride, float *__restrict__ spat,
             long spat_stride) {
   using C = TsF2<P, Q, R>;
@@ -653,7 +658,7 @@ ts_f2_synth(TsFftTab ft, const float2 *__restrict__ fm, long fm_stride, float *_
 
 // spat[field][lat][phi] -> g[field][m][lat].  grid = (ceil(nlat/R), fields).
 template <int P, int Q, int R>
-__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, R))
+__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
 ts_f2_analys(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
              float2 *__restrict__ g, long g_stride) {
   using C = TsF2<P, Q, R>;
@@ -670,7 +675,7 @@ ts_f2_analys(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
 
 // spat[field][lat][phi] -> W image.  grid = (ceil(nh/(R/2)), fields).
 template <int P, int Q, int R>
-__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, R))
+__global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
 ts_f2_analys_w(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
                const float *__restrict__ wq, char *wimg, int nfb, int fpb, int nlc, int nh,
                const int *__restrict__ w_kmin) {

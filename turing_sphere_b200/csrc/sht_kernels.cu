@@ -542,10 +542,16 @@ void f2_analys_w(ts_plan p, const float *spat, long ss, int nf, int fpb, char *w
 }  // namespace
 
 namespace {
-// rows of a standalone FFT CTA: the tuned choice, else the default unless a
-// small batch would leave SMs idle
-int pick_rows(ts_plan p, int nf, int rlo, int rhi) {
+// rows of a standalone FFT CTA: the tuned choice, else the smaller count where
+// the larger would leave SMs idle, and for the 32-point second phase of the
+// synthesis and the plain analysis, which then keep more threads resident (us,
+// 16 | 8 rows: nphi 1536 x 64 fields at lmax 511 178 | 141 and 140 | 133, nphi
+// 1024 x 16 22.8 | 18.4 and 16.7 | 16.7, nphi 2048 x 16 76 | 69 and 60 | 56).
+// The W image wants 8 latitude pairs, whole sectors (154 | 157, 20.4 | 19.6,
+// 64 | 66).
+int pick_rows(ts_plan p, int nf, int P, int rlo, int rhi, bool wimage) {
   if (p->fft_rows) return p->fft_rows == rlo ? rlo : rhi;
+  if (P == 32 && !wimage) return rlo;
   return (long)nf * ((p->nlat + rhi - 1) / rhi) < p->ctx->sm_count ? rlo : rhi;
 }
 }  // namespace
@@ -577,7 +583,7 @@ bool ts_launch_fourier_analys_w(ts_plan p, const float *spat, long ss, int nf, i
   if (p->fourier != TS_FOURIER_FFT) return false;
 #define TS_F2_CASE(h, pp, qq, rlo, rhi)                                     \
   case h:                                                                   \
-    if (pick_rows(p, nf, rlo, rhi) == rlo)                                  \
+    if (pick_rows(p, nf, pp, rlo, rhi, true) == rlo)                                  \
       f2_analys_w<pp, qq, rlo>(p, spat, ss, nf, fpb, wimg, s);              \
     else                                                                    \
       f2_analys_w<pp, qq, rhi>(p, spat, ss, nf, fpb, wimg, s);              \
@@ -600,7 +606,7 @@ void ts_launch_fourier_synth(ts_plan p, const float2 *fm, long fs, float *spat, 
   if (p->fourier == TS_FOURIER_FFT) {
 #define TS_F2_CASE(h, pp, qq, rlo, rhi)                                         \
   case h:                                                                       \
-    return pick_rows(p, nf, rlo, rhi) == rlo ? f2_synth<pp, qq, rlo>(p, fm, fs, spat, ss, nf, s) \
+    return pick_rows(p, nf, pp, rlo, rhi, false) == rlo ? f2_synth<pp, qq, rlo>(p, fm, fs, spat, ss, nf, s) \
                               : f2_synth<pp, qq, rhi>(p, fm, fs, spat, ss, nf, s);
     if (p->fft_alt) switch (p->fft.H) {
         TS_F2_ALT_SHAPES(TS_F2_CASE)
@@ -632,7 +638,7 @@ void ts_launch_fourier_analys(ts_plan p, const float *spat, long ss, float2 *g, 
   if (p->fourier == TS_FOURIER_FFT) {
 #define TS_F2_CASE(h, pp, qq, rlo, rhi)                                        \
   case h:                                                                      \
-    return pick_rows(p, nf, rlo, rhi) == rlo ? f2_analys<pp, qq, rlo>(p, spat, ss, g, gs, nf, s) \
+    return pick_rows(p, nf, pp, rlo, rhi, false) == rlo ? f2_analys<pp, qq, rlo>(p, spat, ss, g, gs, nf, s) \
                               : f2_analys<pp, qq, rhi>(p, spat, ss, g, gs, nf, s);
     if (p->fft_alt) switch (p->fft.H) {
         TS_F2_ALT_SHAPES(TS_F2_CASE)
