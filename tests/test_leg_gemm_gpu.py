@@ -169,3 +169,22 @@ def test_one_and_two_fields(device, parity, precision, lmax, mmax, nlat, nphi):
             worst = max(O.rel_l2(dst[f].cpu().numpy(), y[2 - batch + f]) for f in range(batch))
             parity(f"{precision} lmax{lmax} mmax{mmax} nlat{nlat} B{batch} {name}", worst, TOL)
     plan.destroy()
+
+
+@pytest.mark.parametrize("lmax,nlat,nphi", [(319, 640, 1536), (127, 256, 512), (170, 342, 1024)])
+def test_contraction_repeats_its_bits_on_grids_of_partial_tiles(device, lmax, nlat, nphi):
+    """The tensor-core synthesis where the last latitude tile holds whole chunks
+    and then none: its stores and the staging that follows them must not meet
+    (64 fields, ten calls, the same bits each time, every field alike)."""
+    import torch
+    batch = 64
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": "tf32x3"})
+    src = torch.from_numpy(np.tile(spectrum(lmax, lmax, 3), (batch, 1))).cuda()
+    fm = [torch.empty(batch, 2 * (lmax + 1) * nlat, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    for k in range(10):
+        plan.stage_dev("legSynth", src.data_ptr(), fm[min(k, 1)].data_ptr(), batch)
+        device.sync()
+        assert torch.equal(fm[min(k, 1)], fm[0]), k
+    assert torch.equal(fm[0], fm[0][:1].expand_as(fm[0]))
+    plan.destroy()

@@ -711,6 +711,10 @@ ts_leg_synth_tc(TsLegTab t, TsTcTab tc, const char *__restrict__ qimg, int q_nfb
         sE[ts_syn_stg(et >> 1, 2 * i + (et & 1))] = e[i] + o[i];
         sE[ts_syn_stg(et >> 1, 32 + 2 * i + (et & 1))] = e[i] - o[i];
       }
+      // an empty group: the wait above counts one group per staged chunk, and
+      // would otherwise let the store before this chunk read on while the next
+      // chunk overwrites its buffer
+      if (elected) ts_bulk_commit();
       ts_epi_bar(grp);
 #pragma unroll 2
       for (int k = 0; k < 8; k++) {
