@@ -188,3 +188,29 @@ def test_contraction_repeats_its_bits_on_grids_of_partial_tiles(device, lmax, nl
         assert torch.equal(fm[min(k, 1)], fm[0]), k
     assert torch.equal(fm[0], fm[0][:1].expand_as(fm[0]))
     plan.destroy()
+
+
+@pytest.mark.parametrize("batch", [33, 49])
+def test_first_call_beside_work_on_the_default_stream(device, parity, batch):
+    """A tensor-core plan's first call of a batch clears its new operand images;
+    work queued on the default stream must not put that clearing off until
+    after the kernels that fill them (the context's stream does not wait for
+    the default one)."""
+    import torch
+    lmax, nlat, nphi = 319, 640, 1536
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": "tf32x3"})
+    ref = O.ShtReference(lmax, lmax, nlat, nphi)
+    q = spectrum(lmax, lmax, batch)
+    want = ref.synth(q.astype(np.float64))
+    src = torch.from_numpy(np.tile(q, (batch, 1))).cuda()
+    grid = torch.from_numpy(np.tile(want.astype(np.float32), (batch, 1))).cuda()
+    out = [torch.empty_like(grid), torch.empty_like(src)]
+    for call, x, y in ((plan.synth_dev, src, out[0]), (plan.analys_dev, grid, out[1])):
+        torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)  # some 50 ms on the default stream
+        call(x.data_ptr(), y.data_ptr(), batch)
+        torch.cuda.synchronize()
+    parity(f"tf32x3 lmax319 B{batch} first synth", O.rel_l2(out[0][-1].cpu().numpy(), want), TOL)
+    parity(f"tf32x3 lmax319 B{batch} first analys",
+           O.rel_l2(out[1][-1].cpu().numpy(), ref.analys(want.astype(np.float32).astype(np.float64))), TOL)
+    plan.destroy()

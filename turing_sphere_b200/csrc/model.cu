@@ -1185,6 +1185,7 @@ void adj_prepare(ts_model m) {
       TS_CUDA(cudaLibraryGetKernel(&as.fwd, A.lib, as.fwd_name.c_str()));
       TS_CUDA(cudaLibraryGetKernel(&as.rev, A.lib, as.rev_name.c_str()));
     }
+  TS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the buffers' clearing
   A.ready = true;
 }
 
@@ -1545,6 +1546,9 @@ int ts_model_compile(ts_plan plan, const char *source, const char *const *state,
     m->stash.ensure(sizeof(float) * 2 * nlm * batch * nstate);
     m->h_prm.assign((size_t)std::max(nparams, 1) * batch, 0.0f);
     m->d_prm = dalloc((long)m->h_prm.size());
+    // the buffers were cleared on the default stream, which the context's stream
+    // does not wait for
+    TS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     *out = m;
     return TS_OK;
   } catch (const ts_exc &e) {

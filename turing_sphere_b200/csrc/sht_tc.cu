@@ -556,10 +556,12 @@ __global__ void ts_k_wimage(TsLegTab t, const float2 *g, long gs, int nfields, i
   }
 }
 
-void ensure_zeroed(ts_dbuf &b, size_t bytes) {
+// zeroed on the stream whose kernels write the buffer next: the default stream's
+// memset could run after them (the context's stream does not wait for it)
+void ensure_zeroed(ts_dbuf &b, size_t bytes, cudaStream_t s) {
   if (bytes <= b.cap) return;
   b.ensure(bytes);
-  TS_CUDA(cudaMemset(b.p, 0, b.cap));
+  TS_CUDA(cudaMemsetAsync(b.p, 0, b.cap, s));
 }
 
 }  // namespace
@@ -639,7 +641,7 @@ void ts_launch_leg_synth_tc(ts_plan p, const TsFields &q, float2 *fm, long fs, i
                             cudaStream_t s, ts_dbuf *qbuf) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
   ts_dbuf &b = qbuf ? *qbuf : t->qimg;
-  ensure_zeroed(b, ts_tc_qimg_bytes(p, nf));
+  ensure_zeroed(b, ts_tc_qimg_bytes(p, nf), s);
   ts_launch_qimage(p, q, nf, (char *)b.p, s);
   ts_launch_synth_tc_img(p, (const char *)b.p, nf, fm, fs, s);
 }
@@ -662,7 +664,7 @@ void ts_launch_analys_tc_img(ts_plan p, const char *wimg, int nf, float2 *out, l
 void ts_launch_leg_analys_tc(ts_plan p, const float2 *g, long gs, float2 *out, long os, int nf,
                              cudaStream_t s) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
-  ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS));
+  ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
   ts_launch_wimage(p, g, gs, nf, TS_TC_FIELDS, (char *)t->wimg.p, s);
   ts_launch_analys_tc_img(p, (const char *)t->wimg.p, nf, out, os, s);
 }
@@ -678,7 +680,7 @@ void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf
     ts_launch_leg_analys_gemm(p, (const float2 *)t->gscratch.p, field, (float2 *)qlm, p->nlm, nf, s);
     return;
   }
-  ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS));
+  ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
   if (!ts_launch_fourier_analys_w(p, spat, ss, nf, TS_TC_FIELDS, (char *)t->wimg.p, s)) {
     const long field = (long)(p->mmax + 1) * p->nlat;
     t->gscratch.ensure(sizeof(float2) * field * nf);
