@@ -171,6 +171,40 @@ def test_one_and_two_fields(device, parity, precision, lmax, mmax, nlat, nphi):
     plan.destroy()
 
 
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("batch", [1, 4])
+def test_a_chain_of_small_calls(device, parity, precision, batch):
+    """Calls small enough to launch early (each kernel may start while the one
+    before it runs), 200 round trips back to back over two coefficient buffers
+    and one grid, then the same chain with a wait after every call: the same
+    bits, and the first transform against the oracle."""
+    import torch
+    lmax, nlat, nphi = 63, 96, 192
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": precision})
+    ref = O.ShtReference(lmax, lmax, nlat, nphi)
+    q0 = np.stack([spectrum(lmax, lmax, 11 + k) for k in range(batch)])
+    grid = torch.empty(batch, nlat * nphi, device="cuda")
+
+    def chain(n, wait):
+        a = [torch.from_numpy(q0).cuda(), torch.zeros(q0.shape, device="cuda")]
+        torch.cuda.synchronize()
+        for i in range(n):
+            plan.synth_dev(a[i & 1].data_ptr(), grid.data_ptr(), batch)
+            if wait:
+                device.sync()
+            plan.analys_dev(grid.data_ptr(), a[1 - (i & 1)].data_ptr(), batch)
+            if wait:
+                device.sync()
+        device.sync()
+        return a[n & 1].cpu().numpy(), grid.cpu().numpy()
+
+    first = chain(1, True)
+    parity(f"{precision} lmax63 B{batch} chain synth", O.rel_l2(first[1][0], ref.synth(q0[0].astype(np.float64))), TOL)
+    slow, fast = chain(200, True), chain(200, False)
+    assert np.array_equal(slow[0], fast[0]) and np.array_equal(slow[1], fast[1])
+    plan.destroy()
+
+
 @pytest.mark.parametrize("lmax,nlat,nphi", [(319, 640, 1536), (127, 256, 512), (170, 342, 1024)])
 def test_contraction_repeats_its_bits_on_grids_of_partial_tiles(device, lmax, nlat, nphi):
     """The tensor-core synthesis where the last latitude tile holds whole chunks

@@ -119,6 +119,16 @@ void ts_analys_dev(ts_plan p, const float *spat, float *qlm, int batch, cudaStre
   ts_launch_leg_analys(p, fm, fm_stride, (float2 *)qlm, p->nlm, batch, s);
 }
 
+// Early launches pay while a kernel is shorter than about 5 us; beyond that the
+// waiting CTAs only take room from the running ones.  Pairs (us, FP32 plan, late
+// | early): lmax 63 x 1 17.4 | 11.8, x 4 18.4 | 14.2, lmax 127 x 1 21.5 | 18.4,
+// x 4 (295 K points) 25.8 | 29.9; Schnakenberg steps: lmax 63 x 4 14.7 | 13.3,
+// lmax 127 x 1 (147 K points) 19.4 | 18.5; Allen-Cahn step at lmax 255 25.2 | 27.7.
+// Between the adjoint's other kernels they cost (lmax 127 8 steps 803 | 843).
+bool ts_early(ts_plan p, int nfields) {
+  return !p->no_early && (long)nfields * p->nlat * p->nphi <= 160000;
+}
+
 std::vector<const void *> ts_plan_scratch(ts_plan p) {
   std::vector<const void *> v{p->fm.p, p->adj_grid.p, p->adj_spec.p, p->lg_tab};
   ts_tc_scratch(p, &v);

@@ -637,7 +637,7 @@ constexpr long ts_f2_smem_bytes(int nb) {
 // aligned (fewer, larger memory instructions), else by per-thread stores.
 template <int P, int Q, int R>
 __global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
-ts_f2_synth(TsFftTab ft, const float2 *__restrict__ fm, long fm_stride, float *__restrict__ spat,
+ts_f2_synth(TsFftTab ft, const float2 *fm, long fm_stride, float *spat,
             long spat_stride) {
   using C = TsF2<P, Q, R>;
   extern __shared__ __align__(16) float2 ts_smem_f2s[];
@@ -645,6 +645,8 @@ ts_f2_synth(TsFftTab ft, const float2 *__restrict__ fm, long fm_stride, float *_
   float2 *b = twq + C::TWQ;
   const long f = blockIdx.y;
   const TsF2Rows<C, false> rows{(int)blockIdx.x * R, ft.nlat, 0};
+  ts_grid_go();
+  ts_grid_wait();
   ts_f2_twq<C>(twq, ft);
   ts_f2_pack<C>(b, fm + f * fm_stride, ft, rows);
   __syncthreads();
@@ -659,14 +661,16 @@ ts_f2_synth(TsFftTab ft, const float2 *__restrict__ fm, long fm_stride, float *_
 // spat[field][lat][phi] -> g[field][m][lat].  grid = (ceil(nlat/R), fields).
 template <int P, int Q, int R>
 __global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
-ts_f2_analys(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
-             float2 *__restrict__ g, long g_stride) {
+ts_f2_analys(TsFftTab ft, const float *spat, long spat_stride,
+             float2 *g, long g_stride) {
   using C = TsF2<P, Q, R>;
   extern __shared__ float2 ts_smem_f2a[];
   float2 *twq = ts_smem_f2a;
   float2 *b = twq + C::TWQ;
   const long f = blockIdx.y;
   const TsF2Rows<C, false> rows{(int)blockIdx.x * R, ft.nlat, 0};
+  ts_grid_go();
+  ts_grid_wait();
   ts_f2_twq<C>(twq, ft);
   __syncthreads();
   ts_f2_forward_in<C>(b, twq, spat + f * spat_stride, ft.nphi, rows);
@@ -676,7 +680,7 @@ ts_f2_analys(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
 // spat[field][lat][phi] -> W image.  grid = (ceil(nh/(R/2)), fields).
 template <int P, int Q, int R>
 __global__ void __launch_bounds__(P *R, TS_F2_MINB(P, Q, R))
-ts_f2_analys_w(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
+ts_f2_analys_w(TsFftTab ft, const float *spat, long spat_stride,
                const float *__restrict__ wq, char *wimg, int nfb, int fpb, int nlc, int nh,
                const int *__restrict__ w_kmin) {
   using C = TsF2<P, Q, R>;
@@ -686,6 +690,8 @@ ts_f2_analys_w(TsFftTab ft, const float *__restrict__ spat, long spat_stride,
   const long f = blockIdx.y;
   const int lat0 = blockIdx.x * (R / 2);
   const TsF2Rows<C, true> rows{lat0, ft.nlat, nh};
+  ts_grid_go();
+  ts_grid_wait();
   ts_f2_twq<C>(twq, ft);
   __syncthreads();
   ts_f2_forward_in<C>(b, twq, spat + f * spat_stride, ft.nphi, rows);
@@ -852,6 +858,8 @@ ts_f2_phase(TsFftTab ft, TsPhaseIO io) {
   const long inst = blockIdx.y;
   const int lat0 = blockIdx.x * (PAIRED ? R / 2 : R);
   const TsF2Rows<C, PAIRED> rows{lat0, ft.nlat, io.nh};
+  ts_grid_go();
+  ts_grid_wait();
   ts_f2_twq<C>(twq, ft);
   ts_f2_groups<NSYN, 2>([&](auto s0c, auto nc) {
     constexpr int s0 = decltype(s0c)::value, n = decltype(nc)::value;

@@ -354,6 +354,8 @@ ts_leg_synth_gemm(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ f
   const int par = warp >> 1, cg = lane & 7, rl = (warp & 1) * 32 + (lane >> 3) * 8;
   const float *mt = g.tab + ts_lg_off(t.lmax, m) * g.nhp + lat0;
   const long base = ts_lm_base(t.lmax, m);
+  ts_grid_go();
+  ts_grid_wait();
   for (int f = tid; f < S::NF; f += TS_LG_THREADS)
     src[f] = f0 + f < nfields ? ts_field(q, f0 + f) + base : nullptr;
   if (tid < TS_LG_ROWS) {
@@ -460,7 +462,7 @@ ts_leg_synth_gemm(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ f
 // the first value of a warp's degrees are left out.
 template <int NCOL, class Epi>
 __global__ void __launch_bounds__(TS_LG_THREADS, 4)
-ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, long g_stride, Epi epi,
+ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *gm, long g_stride, Epi epi,
                    int nfields, int per_cta) {
   using S = TsLg<NCOL>;
   extern __shared__ __align__(16) float ts_smem_lg[];
@@ -470,6 +472,8 @@ ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, lo
   const int K = t.lmax - m + 1, kp0 = ts_lg_k16(t.lmax, m, 0), kp1 = ts_lg_k16(t.lmax, m, 1);
   const int nch = (K + 2 * TS_LG_ROWS - 1) / (2 * TS_LG_ROWS);
   if ((int)blockIdx.x >= nch) return;
+  ts_grid_go();
+  ts_grid_wait();
   int per = (((K + 1) >> 1) + nch - 1) / nch;  // degrees of a parity per CTA
   per = per > 32 ? (per + 15) & ~15 : (per + 7) & ~7;
   const int j0 = blockIdx.x * per;
@@ -649,6 +653,14 @@ ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, lo
 // and the columns come as broadcasts from shared memory.  The rows of a CTA are
 // dealt out to its warps, whose sums are added up at the end.
 
+// a load of what the kernel before this one wrote: not through the read-only
+// path, and not moved ahead of ts_grid_wait()
+TS_DEV float2 ts_lg_ld(const float2 *p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
 template <int F>
 TS_DEV void ts_lg_columns(float2 (&c)[F], const float2 *s) {
   if constexpr (F == 1) {
@@ -675,6 +687,8 @@ ts_leg_synth_few(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ fm
   const int lat0 = blockIdx.x * TS_LG_ROWS, m = blockIdx.y, K = t.lmax - m + 1;
   const long base = ts_lm_base(t.lmax, m);
   const int *on = g.onset + (long)m * g.nhp + lat0 + 2 * lane;
+  ts_grid_go();
+  ts_grid_wait();
   const int o0 = __ldg(on), o1 = __ldg(on + 1);
   const float2 *src[F];
 #pragma unroll
@@ -684,7 +698,7 @@ ts_leg_synth_few(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ fm
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
-      for (int f = 0; f < F; f++) v[u][f] = __ldg(src[f] + min(i0 + 256 * u, K - 1));
+      for (int f = 0; f < F; f++) v[u][f] = ts_lg_ld(src[f] + min(i0 + 256 * u, K - 1));
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
@@ -742,13 +756,15 @@ ts_leg_synth_few(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ fm
 // memory: 2 nh F + 16 F 64 float2.
 template <int F, class Epi>
 __global__ void __launch_bounds__(512)
-ts_leg_analys_few(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, long g_stride, Epi epi,
+ts_leg_analys_few(TsLegTab t, TsLegGemmTab g, const float2 *gm, long g_stride, Epi epi,
                   int nfields) {
   extern __shared__ __align__(16) float2 ts_smem_fa[];  // [parity][latitude][F], then [warp][F][64]
   __shared__ int first;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, par = warp & 1, part = warp >> 1;
   const int m = blockIdx.y, j0 = blockIdx.x * TS_LG_ROWS, K = t.lmax - m + 1;
   if (2 * j0 >= K) return;
+  ts_grid_go();
+  ts_grid_wait();
   const int kp0 = ts_lg_k16(t.lmax, m, 0), kp = par ? ts_lg_k16(t.lmax, m, 1) : kp0;
   if (tid == 0) first = t.nh;
   __syncthreads();
@@ -761,8 +777,8 @@ ts_leg_analys_few(TsLegTab t, TsLegGemmTab g, const float2 *__restrict__ gm, lon
       float2 n = make_float2(0.f, 0.f), s = n;
       if (f < nfields) {
         const float2 *src = gm + (long)f * g_stride + (long)m * t.nlat;
-        n = __ldg(src + lat);
-        if (south != lat) s = __ldg(src + south);
+        n = ts_lg_ld(src + lat);
+        if (south != lat) s = ts_lg_ld(src + south);
       }
       ts_smem_fa[lat * F + f] = c_scale(c_add(n, s), w);
       ts_smem_fa[(t.nh + lat) * F + f] = c_scale(c_sub(n, s), w);

@@ -21,6 +21,16 @@
 // a >= b ? x : y (derivatives of max/min in generated adjoint code)
 TS_DEV float ts_ge_sel(float a, float b, float x, float y) { return a >= b ? x : y; }
 
+// Programmatic dependent launch: a kernel launched with it (ts_launch) may start
+// while the kernel before it in the stream still runs, once all of that one's
+// CTAs have said ts_grid_go() (or ended).  ts_grid_wait() returns when that
+// kernel has ended and its writes are visible; before it a kernel touches
+// nothing, and what that kernel may have written is not read through the
+// read-only path.  As every kernel waits before it ends, the one after it finds
+// all earlier ones ended too.  Launched without it, both do nothing.
+TS_DEV void ts_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+TS_DEV void ts_grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 TS_DEV float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 TS_DEV float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 TS_DEV float2 c_scale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }

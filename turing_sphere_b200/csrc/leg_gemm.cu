@@ -62,7 +62,7 @@ void synth_t(ts_plan p, const TsLegGemmTab &g, const TsFields &q, float2 *fm, lo
   using S = TsLg<NCOL>;
   ts_allow_smem((const void *)ts_leg_synth_gemm<NCOL>, p->ctx->device, S::SYN_SMEM);
   dim3 grid(g.nhp / TS_LG_ROWS, (nf + S::NF - 1) / S::NF, p->mmax + 1);
-  ts_leg_synth_gemm<NCOL><<<grid, TS_LG_THREADS, S::SYN_SMEM, s>>>(p->leg, g, q, fm, fs, nf);
+  ts_launch(ts_early(p, nf), ts_leg_synth_gemm<NCOL>, grid, TS_LG_THREADS, S::SYN_SMEM, s, p->leg, g, q, fm, fs, nf);
 }
 
 template <int NCOL>
@@ -72,7 +72,7 @@ void analys_t(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, const
   const auto kernel = ts_leg_analys_gemm<NCOL, TsLgStore>;
   ts_allow_smem((const void *)kernel, p->ctx->device, S::ANA_SMEM);
   dim3 grid((p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS), (nf + S::NF - 1) / S::NF, p->mmax + 1);
-  kernel<<<grid, TS_LG_THREADS, S::ANA_SMEM, s>>>(p->leg, g, gm, gs, out, nf, S::NF);
+  ts_launch(ts_early(p, nf), kernel, grid, TS_LG_THREADS, S::ANA_SMEM, s, p->leg, g, gm, gs, out, nf, (int)S::NF);
 }
 
 template <int F>
@@ -80,7 +80,7 @@ void synth_few(ts_plan p, const TsLegGemmTab &g, const TsFields &q, float2 *fm, 
                cudaStream_t s) {
   const size_t smem = sizeof(float2) * (size_t)(p->lmax + 1) * F;
   ts_allow_smem((const void *)ts_leg_synth_few<F>, p->ctx->device, smem);
-  ts_leg_synth_few<F><<<dim3(g.nhp / TS_LG_ROWS, p->mmax + 1), 256, smem, s>>>(p->leg, g, q, fm, fs, nf);
+  ts_launch(ts_early(p, nf), ts_leg_synth_few<F>, dim3(g.nhp / TS_LG_ROWS, p->mmax + 1), 256, smem, s, p->leg, g, q, fm, fs, nf);
 }
 
 size_t few_smem(ts_plan p, int F) { return sizeof(float2) * F * (2 * (size_t)p->nh + 16 * TS_LG_ROWS); }
@@ -91,7 +91,7 @@ void analys_few(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, con
   const auto kernel = ts_leg_analys_few<F, TsLgStore>;
   ts_allow_smem((const void *)kernel, p->ctx->device, few_smem(p, F));
   dim3 grid((p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS), p->mmax + 1);
-  kernel<<<grid, 512, few_smem(p, F), s>>>(p->leg, g, gm, gs, out, nf);
+  ts_launch(ts_early(p, nf), kernel, grid, 512, few_smem(p, F), s, p->leg, g, gm, gs, out, nf);
 }
 
 // One or two fields take the kernels without staging (us, tiled | these, lmax

@@ -867,7 +867,8 @@ void run_program(ts_model m, Program &P, cudaStream_t st) {
         if (s.threads) {  // two-phase FFT: R rows (R/2 latitude pairs) per CTA
           const int per = s.wimg ? s.lb / 2 : s.lb;
           dim3 grid(((s.wimg ? p->nh : p->nlat) + per - 1) / per, B);
-          TS_CUDA(cudaLaunchKernel((const void *)s.kern, grid, dim3(s.threads), args, s.smem, st));
+          ts_launch_args(ts_early(p, B * std::max(s.nsyn, s.nana)), (const void *)s.kern, grid, dim3(s.threads),
+                         s.smem, st, args);
         } else {
           dim3 grid((p->nlat + s.lb - 1) / s.lb, B);
           TS_CUDA(cudaLaunchKernel((const void *)s.kern, grid, dim3(32 * s.lb), args, s.smem, st));
@@ -886,8 +887,8 @@ void run_program(ts_model m, Program &P, cudaStream_t st) {
         if (s.lg.threads) {
           TsLegGemmTab tab = p->lg_ana;
           void *args[] = {&leg, &tab, &g, &gs, &epi, &nfields, &per_cta};  // (few: without per_cta)
-          TS_CUDA(cudaLaunchKernel((const void *)s.kern, dim3(s.lg.grid[0], s.lg.grid[1], s.lg.grid[2]),
-                                   dim3(s.lg.threads), args, s.smem, st));
+          ts_launch_args(ts_early(p, nfields), (const void *)s.kern, dim3(s.lg.grid[0], s.lg.grid[1], s.lg.grid[2]),
+                         dim3(s.lg.threads), s.smem, st, args);
         } else if (p->precision != TS_PREC_FP32) {
           TsTcTab tc = ts_tc_tab(p);
           int S = ts_tc_analys_stages(p);
@@ -1258,9 +1259,16 @@ void axpy(float *y, const float *x, long n, cudaStream_t st) {
   TS_CUDA(cudaGetLastError());
 }
 
+struct NoEarly {  // launches of this scope do not start early
+  ts_plan p;
+  explicit NoEarly(ts_plan p_) : p(p_) { p->no_early = true; }
+  ~NoEarly() { p->no_early = false; }
+};
+
 // the step's values from the states at `states[s]` ([instance][2 nlm] each)
 void adj_tape(ts_model m, const std::vector<const float *> &states, cudaStream_t st) {
   Adjoint &A = m->adj;
+  const NoEarly late(m->plan);
   const tsm::Function &f = m->prog[1].fn;
   const int B = m->batch;
   for (size_t s = 0; s < states.size(); s++) A.val[A.state_in[s]] = const_cast<float *>(states[s]);
@@ -1283,6 +1291,7 @@ void adj_tape(ts_model m, const std::vector<const float *> &states, cudaStream_t
 // cotangent of its input state s out (in place); parameter gradients add up
 void adj_reverse(ts_model m, const std::vector<float *> &lam, cudaStream_t st) {
   Adjoint &A = m->adj;
+  const NoEarly late(m->plan);
   const tsm::Function &f = m->prog[1].fn;
   const int B = m->batch;
   for (size_t v = 0; v < A.bar.size(); v++)

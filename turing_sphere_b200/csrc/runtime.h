@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/turing_sht.h"
@@ -30,6 +31,37 @@ struct ts_exc {
   do {                              \
     if (!(cond)) ts_throw(code, msg); \
   } while (0)
+
+// Launches a kernel that, with `early`, may start while the kernel before it in the
+// stream still runs (programmatic dependent launch): it calls ts_grid_wait() before it
+// touches anything.  A small call is a chain of kernels of
+// a few microseconds, and each one's launch and prologue then overlap the one
+// before it.
+inline void ts_launch_args(bool early, const void *kernel, dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t s, void **args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  TS_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+}
+template <class... P, class... A>
+void ts_launch(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+               A... a) {
+  std::tuple<P...> v(a...);
+  std::apply(
+      [&](P &...x) {
+        void *args[] = {(void *)&x...};
+        ts_launch_args(early, (const void *)kernel, grid, block, smem, s, args);
+      },
+      v);
+}
 
 // Device arrays of the transforms hold complex pairs and grid rows that the
 // kernels read and write as float2 (8 bytes); a float pointer that is only
@@ -123,7 +155,10 @@ struct ts_plan_s {
   // the FFT's second P*Q split (TS_F2_ALT_SHAPES) instead of the default one
   bool fft_alt = false;
   bool tuned = false;
+  bool no_early = false;  // set while the adjoint launches (see ts_early)
 };
+
+bool ts_early(ts_plan p, int nfields);  // whether a call of that size launches early
 
 // whole transforms on device buffers (capi.cu) and their adjoints (adjoint.cu)
 void ts_synth_dev(ts_plan p, const float *qlm, float *spat, int batch, cudaStream_t s);

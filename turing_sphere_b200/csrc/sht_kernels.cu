@@ -516,7 +516,7 @@ void f2_synth(ts_plan p, const float2 *fm, long fs, float *spat, long ss, int nf
   const size_t smem = ts_f2_bytes(P, Q, R, 1);
   ts_allow_smem((const void *)ts_f2_synth<P, Q, R>, p->ctx->device, smem);
   dim3 grid((p->nlat + R - 1) / R, nf);
-  ts_f2_synth<P, Q, R><<<grid, P * R, smem, s>>>(p->fft, fm, fs, spat, ss);
+  ts_launch(ts_early(p, nf), ts_f2_synth<P, Q, R>, grid, P * R, smem, s, p->fft, fm, fs, spat, ss);
   TS_CUDA(cudaGetLastError());
 }
 template <int P, int Q, int R>
@@ -524,7 +524,7 @@ void f2_analys(ts_plan p, const float *spat, long ss, float2 *g, long gs, int nf
   const size_t smem = ts_f2_bytes(P, Q, R, 1);
   ts_allow_smem((const void *)ts_f2_analys<P, Q, R>, p->ctx->device, smem);
   dim3 grid((p->nlat + R - 1) / R, nf);
-  ts_f2_analys<P, Q, R><<<grid, P * R, smem, s>>>(p->fft, spat, ss, g, gs);
+  ts_launch(ts_early(p, nf), ts_f2_analys<P, Q, R>, grid, P * R, smem, s, p->fft, spat, ss, g, gs);
   TS_CUDA(cudaGetLastError());
 }
 template <int P, int Q, int R>
@@ -534,9 +534,8 @@ void f2_analys_w(ts_plan p, const float *spat, long ss, int nf, int fpb, char *w
   ts_allow_smem((const void *)ts_f2_analys_w<P, Q, R>, p->ctx->device, smem);
   const int nlc = (p->nh + 31) / 32;
   dim3 grid((p->nh + R / 2 - 1) / (R / 2), nf);
-  ts_f2_analys_w<P, Q, R><<<grid, P * R, smem, s>>>(p->fft, spat, ss, p->d_wq, wimg,
-                                                    (nf + fpb - 1) / fpb, fpb, nlc, p->nh,
-                                                    ts_tc_w_kmin(p));
+  ts_launch(ts_early(p, nf), ts_f2_analys_w<P, Q, R>, grid, P * R, smem, s, p->fft, spat, ss, p->d_wq, wimg,
+            (nf + fpb - 1) / fpb, fpb, nlc, p->nh, ts_tc_w_kmin(p));
   TS_CUDA(cudaGetLastError());
 }
 }  // namespace
