@@ -126,7 +126,7 @@ void ts_analys_dev(ts_plan p, const float *spat, float *qlm, int batch, cudaStre
 // lmax 127 x 1 (147 K points) 19.4 | 18.5; Allen-Cahn step at lmax 255 25.2 | 27.7.
 // Between the adjoint's other kernels they cost (lmax 127 8 steps 803 | 843).
 bool ts_early(ts_plan p, int nfields) {
-  return !p->no_early && (long)nfields * p->nlat * p->nphi <= 160000;
+  return !p->in_adjoint && (long)nfields * p->nlat * p->nphi <= 160000;
 }
 
 std::vector<const void *> ts_plan_scratch(ts_plan p) {

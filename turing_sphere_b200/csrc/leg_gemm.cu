@@ -125,11 +125,19 @@ bool lg_few(int nf) { return nf <= 2; }
 // so the line lies at 16 fields, or for the synthesis at 48 where the table
 // stays in the L2 and 32 up to 256 MB, and for the smallest analyses at 48.
 // No table above 2 GB or lmax 1535.
+//
+// Not in a model's adjoint: a parameter's gradient can be a difference of large
+// terms (the derivative to dt sums the rate of change, A - (B + 1) u + u u v at
+// a Brusselator's steady state), so the contraction's 1e-6 is up to 4e-4 of it
+// (lmax 235) and the gradient of an instance would change by as much with the
+// number of instances beside it.
 bool ts_lg_use(ts_plan p, int nf, bool analysis) {
   const size_t bytes = lg_bytes(p);
   if (!lg_fits(p)) return false;
   if (p->precision != TS_PREC_FP32) {
-    if (ts_tc_stalled(p)) return false;  // the test hook is about the tensor-core kernels
+    // the adjoint of a model takes the contraction whatever the batch; the test
+    // hook is about the tensor-core kernels
+    if (p->in_adjoint || ts_tc_stalled(p)) return false;
     if (analysis) return nf <= (bytes < (size_t)2 << 20 ? 48 : 16);
     return nf <= (bytes <= (size_t)64 << 20 ? 48 : bytes <= (size_t)256 << 20 ? 32 : 16);
   }

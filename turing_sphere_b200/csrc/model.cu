@@ -1259,16 +1259,26 @@ void axpy(float *y, const float *x, long n, cudaStream_t st) {
   TS_CUDA(cudaGetLastError());
 }
 
-struct NoEarly {  // launches of this scope do not start early
+struct AdjointScope {  // launches of this scope are the adjoint's
   ts_plan p;
-  explicit NoEarly(ts_plan p_) : p(p_) { p->no_early = true; }
-  ~NoEarly() { p->no_early = false; }
+  explicit AdjointScope(ts_plan p_) : p(p_) { p->in_adjoint = true; }
+  ~AdjointScope() { p->in_adjoint = false; }
 };
+
+// whether a step's transforms are, in part, the FP32 products of a small batch
+// on a tensor-core plan, and so not those of its adjoint
+bool step_takes_products(ts_model m) {
+  if (m->plan->precision == TS_PREC_FP32) return false;
+  for (auto &s : m->prog[1].stages)
+    if (s.lg.threads || (s.kind == Stage::LegSynth && ts_lg_use(m->plan, m->batch * s.nsyn, false)))
+      return true;
+  return false;
+}
 
 // the step's values from the states at `states[s]` ([instance][2 nlm] each)
 void adj_tape(ts_model m, const std::vector<const float *> &states, cudaStream_t st) {
   Adjoint &A = m->adj;
-  const NoEarly late(m->plan);
+  const AdjointScope scope(m->plan);
   const tsm::Function &f = m->prog[1].fn;
   const int B = m->batch;
   for (size_t s = 0; s < states.size(); s++) A.val[A.state_in[s]] = const_cast<float *>(states[s]);
@@ -1291,7 +1301,7 @@ void adj_tape(ts_model m, const std::vector<const float *> &states, cudaStream_t
 // cotangent of its input state s out (in place); parameter gradients add up
 void adj_reverse(ts_model m, const std::vector<float *> &lam, cudaStream_t st) {
   Adjoint &A = m->adj;
-  const NoEarly late(m->plan);
+  const AdjointScope scope(m->plan);
   const tsm::Function &f = m->prog[1].fn;
   const int B = m->batch;
   for (size_t v = 0; v < A.bar.size(); v++)
@@ -1853,14 +1863,6 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   A.cur.ensure(sizeof(float) * sz * ns);
   float *pck = (float *)A.ck.p, *pseg = (float *)A.seg.p, *plam = (float *)A.lam.p,
         *pcur = (float *)A.cur.p;
-  for (int i = 0; i < nsteps; i += every) {
-    for (int s = 0; s < ns; s++)
-      TS_CUDA(cudaMemcpyAsync(pck + ((long)(i / every) * ns + s) * sz, m->host.at(m->state[s]).cur,
-                              sizeof(float) * sz, cudaMemcpyDeviceToDevice, st));
-    advance(m, std::min(every, nsteps - i));
-  }
-  TS_CUDA(cudaMemcpyAsync(plam, final_bar, sizeof(float) * sz * ns, cudaMemcpyHostToDevice, st));
-  TS_CUDA(cudaMemsetAsync(A.pbar, 0, sizeof(double) * std::max<size_t>(m->params.size(), 1) * B, st));
   std::vector<float *> lam(ns);
   std::vector<const float *> cur(ns);
   for (int s = 0; s < ns; s++) {
@@ -1870,17 +1872,42 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   auto copy = [&](float *dst, const float *src) {
     TS_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * sz * ns, cudaMemcpyDeviceToDevice, st));
   };
+  auto take_state = [&](float *dst) {  // the model's current states
+    for (int s = 0; s < ns; s++)
+      TS_CUDA(cudaMemcpyAsync(dst + (long)s * sz, m->host.at(m->state[s]).cur, sizeof(float) * sz,
+                              cudaMemcpyDeviceToDevice, st));
+  };
+  auto replay_step = [&] {  // the states in `cur` one step on
+    adj_graphed(m, &A.fwd_graph, st, [&] {
+      adj_tape(m, cur, st);
+      for (int s = 0; s < ns; s++)
+        TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
+                                cudaMemcpyDeviceToDevice, st));
+    });
+  };
+  if (nseg > 1 && step_takes_products(m)) {
+    // the checkpoints lie on the adjoint's own trajectory, which the step's
+    // products would leave by their difference to the contraction
+    take_state(pcur);
+    for (int g = 0; g < nseg; g++) {
+      copy(pck + (long)g * ns * sz, pcur);
+      for (int j = 0; j < every && g + 1 < nseg; j++) replay_step();
+    }
+    advance(m, nsteps);
+  } else {
+    for (int i = 0; i < nsteps; i += every) {
+      take_state(pck + (long)(i / every) * ns * sz);
+      advance(m, std::min(every, nsteps - i));
+    }
+  }
+  TS_CUDA(cudaMemcpyAsync(plam, final_bar, sizeof(float) * sz * ns, cudaMemcpyHostToDevice, st));
+  TS_CUDA(cudaMemsetAsync(A.pbar, 0, sizeof(double) * std::max<size_t>(m->params.size(), 1) * B, st));
   for (int g = nseg - 1; g >= 0; g--) {
     const int len = std::min(every, nsteps - g * every);
     copy(pcur, pck + (long)g * ns * sz);
     copy(pseg, pcur);
     for (int j = 1; j < len; j++) {  // replay the segment: the state before every step
-      adj_graphed(m, &A.fwd_graph, st, [&] {
-        adj_tape(m, cur, st);
-        for (int s = 0; s < ns; s++)
-          TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
-                                  cudaMemcpyDeviceToDevice, st));
-      });
+      replay_step();
       copy(pseg + (long)j * ns * sz, pcur);
     }
     for (int j = len - 1; j >= 0; j--) {

@@ -155,7 +155,7 @@ struct ts_plan_s {
   // the FFT's second P*Q split (TS_F2_ALT_SHAPES) instead of the default one
   bool fft_alt = false;
   bool tuned = false;
-  bool no_early = false;  // set while the adjoint launches (see ts_early)
+  bool in_adjoint = false;  // set while a model's adjoint launches (see ts_early, ts_lg_use)
 };
 
 bool ts_early(ts_plan p, int nfields);  // whether a call of that size launches early
