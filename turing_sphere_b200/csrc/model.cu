@@ -510,7 +510,8 @@ void schedule(ts_model m, Program &P, bool is_step) {
       int fP = 0, fQ = 0, fR = 0;
       const int nb = std::max<int>({(int)S.size(), (int)A.size(), 1});
       if (ts_f2_phase_shape(p, &fP, &fQ)) fR = ts_f2_phase_rows(p, nb, m->batch, &st.smem);
-      lg = !A.empty() && ts_lg_use(p, m->batch * (int)A.size(), true) &&
+      // the smallest tile of the products holds 8 fields, whole instances
+      lg = !A.empty() && A.size() <= 8 && ts_lg_use(p, m->batch * (int)A.size(), true) &&
            (m->host_only || ts_lg_prepare(p, m->ctx->stream));
       const bool tcw = p->precision != TS_PREC_FP32 && !lg && fR && !A.empty();
       if (fR) {
