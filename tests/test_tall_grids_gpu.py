@@ -1,0 +1,34 @@
+"""Grids with many latitudes, where the shared memory of the kernels for one
+and two fields (16 bytes a latitude and field) comes to its limits."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from turing_sphere_b200 import (GpuModel, ShtConfig, ShtPlan, defaultParams, mModelByKey,
+                                seededNoise)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("nlat", [1024, 2047, 2048])
+def test_one_instance_of_two_species(device, parity, precision, nlat):
+    """At 2047 and 2048 latitudes the analysis asks for exactly 48 KB beside
+    its static shared memory.  Three steps against the oracle (the relative L2
+    bound of the model tests, 1e-4)."""
+    lmax, nphi, steps = 31, 64, 3
+    model = mModelByKey("schnakenberg")
+    p = defaultParams(model)
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": precision})
+    gpu = GpuModel.create(device, plan, model.source, [k.key for k in model.params], model.state,
+                          model.species, 1)
+    gpu.setParams(p)
+    gpu.init(seededNoise(nlat * nphi, model.seedAmp, 1))
+    st0 = [gpu.read(s) for s in model.state]
+    gpu.step(steps)
+    want = O.ShtReference(lmax, lmax, nlat, nphi).model_step(
+        "schnakenberg", [np.float32(p[k.key]) for k in model.params], np.stack(st0).astype(np.float64), steps)
+    for i, name in enumerate(model.state):
+        parity(f"{precision} schnakenberg lmax31 nlat{nlat} {name}", O.rel_l2(gpu.read(name), want[i]), 1e-4)
+    gpu.destroy()
+    plan.destroy()

@@ -795,7 +795,8 @@ void compile_kernels(ts_model m) {
       const std::string name = lowered.count(s.expr) ? lowered[s.expr] : s.expr;
       TS_CUDA(cudaLibraryGetKernel(&s.kern, m->lib, name.c_str()));
       if (!s.expr_v4.empty()) TS_CUDA(cudaLibraryGetKernel(&s.kern_v4, m->lib, s.expr_v4.c_str()));
-      if (s.smem > 48 * 1024)
+      // (the 48 KB that need no attribute hold a kernel's static shared memory too)
+      if (s.smem > 32 * 1024)
         TS_CUDA(cudaKernelSetAttributeForDevice(
             s.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem, m->ctx->device));
     }
