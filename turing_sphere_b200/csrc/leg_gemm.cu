@@ -98,7 +98,12 @@ void analys_few(ts_plan p, const TsLegGemmTab &g, const float2 *gm, long gs, con
 // 255: synthesis 1 field 12.5 | 9.2, 2: 12.6 | 10.5, 4: 12.5 | 12.7; analysis 1:
 // 16.8 | 10.4, 2: 16.8 | 10.5, 4: 17.4 | 14.7; lmax 1023, whole transforms:
 // synthesis 1: 343 | 222, 4: 389 | 426; analysis 1: 382 | 252, 4: 425 | 486).
+// Their analysis holds the columns of every latitude in shared memory: up to
+// some 13500 latitudes for two fields and 28000 for one.
 bool lg_few(int nf) { return nf <= 2; }
+bool lg_few_analys(ts_plan p, int nf) {
+  return lg_few(nf) && few_smem(p, nf) + 64 <= p->ctx->smem_optin;  // (64: the static part)
+}
 
 }  // namespace
 
@@ -198,7 +203,7 @@ bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *gm, long gs, float2 *out
   st.base[0] = out;
   st.inst_stride[0] = os;
   st.nper = 1;
-  if (lg_few(nf))
+  if (lg_few_analys(p, nf))
     nf == 1 ? analys_few<1>(p, g, gm, gs, st, nf, s) : analys_few<2>(p, g, gm, gs, st, nf, s);
   else switch (lg_ncol(nf, 1)) {
     case 64: analys_t<64>(p, g, gm, gs, st, nf, s); break;
@@ -213,7 +218,7 @@ bool ts_lg_prepare(ts_plan p, cudaStream_t s) { return lg_ready(p, s); }
 
 void ts_lg_analys_shape(ts_plan p, int nf, int na, TsLgShape *sh) {
   const unsigned chunks = (p->lmax + 2 * TS_LG_ROWS) / (2 * TS_LG_ROWS), M = p->mmax + 1;
-  if (lg_few(nf)) {
+  if (lg_few_analys(p, nf)) {
     sh->few = nf;
     sh->per_cta = nf;
     sh->threads = 512;
