@@ -288,6 +288,10 @@ int ts_model_group_destroy(ts_group group);
  * dL/d(parameters), host double [instance][nparams]. */
 int ts_model_forward_backward(ts_model model, int nsteps, int every, const float *final_bar,
                               float *init_bar, double *param_bar);
+/* The adjoint's steps run as CUDA graphs too, each kind after two eager ones:
+ * how many replayed and reverse steps of this model did so far (either may be
+ * NULL).  enable = 0 of ts_model_set_graphs runs them eagerly. */
+int ts_model_adjoint_graphs(ts_model model, long *replayed, long *reverse);
 
 /* GpuModel.read (model.ts:262-277): blocking read of a named value — from the
  * function that ran most recently, as #locate does (model.ts:243-252).

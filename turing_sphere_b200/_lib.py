@@ -114,6 +114,7 @@ SIGNATURES = {
     "ts_model_step": (i32, [vp, i32]),
     "ts_model_set_graphs": (i32, [vp, i32]),
     "ts_model_forward_backward": (i32, [vp, i32, i32, f32p, f32p, f64p]),
+    "ts_model_adjoint_graphs": (i32, [vp, C.POINTER(i64), C.POINTER(i64)]),
     "ts_model_group_create": (i32, [C.POINTER(vp), i32, C.POINTER(vp)]),
     "ts_model_group_step": (i32, [vp, i32]),
     "ts_model_group_destroy": (i32, [vp]),

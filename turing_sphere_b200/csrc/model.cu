@@ -172,6 +172,16 @@ struct AdjStmt {
   std::vector<int> in;       // value inputs, in the order of TsAdjIO::in
   std::vector<int> dvars;    // inputs that receive cotangents (TsAdjIO::gin)
 };
+// A kind of the adjoint's steps as a graph.  It holds pointers into the plan's
+// scratch (`key`) and is captured again when that has moved.
+struct AdjGraph {
+  cudaGraphExec_t exec = nullptr;
+  std::vector<const void *> key;
+  int eager_left = 2;  // steps of this kind that run eagerly first: they size the scratch
+  bool ok = true;      // false once a capture has failed with all scratch in place
+  long launched = 0;
+};
+
 struct Adjoint {
   bool ready = false;
   cudaLibrary_t lib = nullptr;
@@ -188,12 +198,8 @@ struct Adjoint {
   // [state] and the states a tape starts from, kept from call to call
   ts_dbuf ck, seg, lam, cur;
   // one replayed step (tape, its final states to `cur`) and one reverse step
-  // (tape, adjoint) as graphs; they hold pointers into the plan's scratch, so
-  // they are dropped when that has moved since the capture
-  cudaGraphExec_t fwd_graph = nullptr, rev_graph = nullptr;
-  std::vector<const void *> key;
-  int eager_left = 4;  // steps of each kind run eagerly first (scratch then has its size)
-  bool graphs_ok = true;
+  // (tape, adjoint) as graphs
+  AdjGraph fwd, rev;
 };
 
 struct ts_model_s {
@@ -1193,9 +1199,9 @@ void adj_prepare(ts_model m) {
 }
 
 void adj_drop_graphs(Adjoint &A) {
-  for (cudaGraphExec_t *g : {&A.fwd_graph, &A.rev_graph}) {
-    if (*g) cudaGraphExecDestroy(*g);
-    *g = nullptr;
+  for (AdjGraph *g : {&A.fwd, &A.rev}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    g->exec = nullptr;
   }
 }
 
@@ -1339,23 +1345,22 @@ std::vector<const void *> adj_key(ts_model m) {
   return k;
 }
 
-// `run` (only launches, copies and memsets on `st`) by way of the graph in
-// *exec, captured on first use; eagerly when graphs are off, cannot be used on
-// this stream or fail to capture, and for the first steps
+// `run` (only launches, copies and memsets on `st`) by way of the graph `g`,
+// captured on first use; eagerly for the first steps of its kind, when graphs
+// are off or cannot be used on this stream, and when the capture fails
 template <class F>
-void adj_graphed(ts_model m, cudaGraphExec_t *exec, cudaStream_t st, F &&run) {
-  Adjoint &A = m->adj;
-  if (A.eager_left > 0 || !A.graphs_ok || !graphs_usable(m)) {
-    if (A.eager_left > 0) A.eager_left--;
+void adj_graphed(ts_model m, AdjGraph &g, cudaStream_t st, F &&run) {
+  if (g.eager_left > 0 || !g.ok || !graphs_usable(m)) {
     run();
+    if (g.eager_left > 0) g.eager_left--;
     return;
   }
   const std::vector<const void *> key = adj_key(m);
-  if (key != A.key) {
-    adj_drop_graphs(A);
-    A.key = key;
+  if (g.exec && key != g.key) {
+    cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
   }
-  if (!*exec) {
+  if (!g.exec) {
     cudaGraph_t graph = nullptr;
     bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
@@ -1365,20 +1370,22 @@ void adj_graphed(ts_model m, cudaGraphExec_t *exec, cudaStream_t st, F &&run) {
         ok = false;
       }
       const bool ended = cudaStreamEndCapture(st, &graph) == cudaSuccess;
-      ok = ok && ended && graph && adj_key(m) == key;
+      ok = ok && ended && graph;
     }
-    if (ok) ok = cudaGraphInstantiate(exec, graph, 0) == cudaSuccess;
+    const bool moved = adj_key(m) != key;  // scratch grew: the next step has it in place
+    if (ok && !moved) ok = cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
     if (graph) cudaGraphDestroy(graph);
-    if (!ok) {
+    if (!ok || moved) {
       (void)cudaGetLastError();
-      *exec = nullptr;
-      A.graphs_ok = false;
-      adj_drop_graphs(A);
+      g.exec = nullptr;
+      if (!moved) g.ok = false;
       run();
       return;
     }
+    g.key = key;
   }
-  TS_CUDA(cudaGraphLaunch(*exec, st));
+  TS_CUDA(cudaGraphLaunch(g.exec, st));
+  g.launched++;
 }
 
 void free_model(ts_model m) {
@@ -1880,7 +1887,7 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
                               cudaMemcpyDeviceToDevice, st));
   };
   auto replay_step = [&] {  // the states in `cur` one step on
-    adj_graphed(m, &A.fwd_graph, st, [&] {
+    adj_graphed(m, A.fwd, st, [&] {
       adj_tape(m, cur, st);
       for (int s = 0; s < ns; s++)
         TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
@@ -1914,7 +1921,7 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
     }
     for (int j = len - 1; j >= 0; j--) {
       if (j < len - 1) copy(pcur, pseg + (long)j * ns * sz);
-      adj_graphed(m, &A.rev_graph, st, [&] {
+      adj_graphed(m, A.rev, st, [&] {
         adj_tape(m, cur, st);
         adj_reverse(m, lam, st);
       });
@@ -1936,6 +1943,13 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
     A.lam.release();
     A.cur.release();
   }
+  TSM_END
+}
+
+int ts_model_adjoint_graphs(ts_model m, long *replayed, long *reverse) {
+  TSM_BEGIN(m)
+  if (replayed) *replayed = m->adj.fwd.launched;
+  if (reverse) *reverse = m->adj.rev.launched;
   TSM_END
 }
 
