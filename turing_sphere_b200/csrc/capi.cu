@@ -119,6 +119,13 @@ void ts_analys_dev(ts_plan p, const float *spat, float *qlm, int batch, cudaStre
   ts_launch_leg_analys(p, fm, fm_stride, (float2 *)qlm, p->nlm, batch, s);
 }
 
+bool ts_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
+}
+
 // Early launches pay while a kernel is shorter than about 5 us; beyond that the
 // waiting CTAs only take room from the running ones.  Pairs (us, FP32 plan, late
 // | early): lmax 63 x 1 17.4 | 11.8, x 4 18.4 | 14.2, lmax 127 x 1 21.5 | 18.4,

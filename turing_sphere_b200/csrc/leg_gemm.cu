@@ -24,11 +24,7 @@ bool lg_fits(ts_plan p) {
 bool lg_ready(ts_plan p, cudaStream_t s) {
   if (p->lg_tab) return true;
   if (p->precision == TS_PREC_FP32) return false;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    (void)cudaGetLastError();
-    return false;
-  }
+  if (ts_capturing(s)) return false;
   ts_lg_init(p, s);
   if (p->lg_tab) TS_CUDA(cudaStreamSynchronize(s));  // later calls may come on other streams
   return p->lg_tab != nullptr;

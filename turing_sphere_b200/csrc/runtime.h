@@ -158,6 +158,7 @@ struct ts_plan_s {
   bool in_adjoint = false;  // set while a model's adjoint launches (see ts_early, ts_lg_use)
 };
 
+bool ts_capturing(cudaStream_t s);  // or its state cannot be told: nothing may be allocated
 bool ts_early(ts_plan p, int nfields);  // whether a call of that size launches early
 
 // whole transforms on device buffers (capi.cu) and their adjoints (adjoint.cu)
@@ -249,6 +250,11 @@ struct TsTcGeom {
 TsTcGeom ts_tc_geom(ts_plan p);
 void ts_tc_set_fault(ts_plan p, int stall_copies, unsigned wait_limit);
 bool ts_tc_stalled(ts_plan p);
+// the operand image that the contraction of nf fields would fill: a call that
+// takes the FP32 products sizes it too, so that a call of more fields can be
+// captured after it (not while the stream is being captured)
+void ts_tc_size_qimg(ts_plan p, int nf, cudaStream_t s);
+void ts_tc_size_wimg(ts_plan p, int nf, cudaStream_t s);
 void ts_tc_scratch(ts_plan p, std::vector<const void *> *out);
 // tiles / chunks the tensor-core polar skip drops
 void ts_tc_skip_counts(ts_plan p, int *tiles, int *chunks);

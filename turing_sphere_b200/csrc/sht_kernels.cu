@@ -371,7 +371,7 @@ void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long f
   qf.base[0] = q;
   qf.inst_stride[0] = qs;
   qf.nper = 1;
-  if (ts_launch_leg_synth_gemm(p, qf, fm, fs, nf, s)) return;
+  if (ts_launch_leg_synth_gemm(p, qf, fm, fs, nf, s)) return ts_tc_size_qimg(p, nf, s);
   if (p->precision != TS_PREC_FP32) return ts_launch_leg_synth_tc(p, qf, fm, fs, nf, s);
   if (nf >= 8) return leg_synth_t<8>(p, q, qs, fm, fs, nf, s);
   if (nf >= 4) return leg_synth_t<4>(p, q, qs, fm, fs, nf, s);
@@ -381,7 +381,7 @@ void ts_launch_leg_synth(ts_plan p, const float2 *q, long qs, float2 *fm, long f
 
 void ts_launch_leg_analys(ts_plan p, const float2 *g, long gs, float2 *q, long qs, int nf,
                           cudaStream_t s) {
-  if (ts_launch_leg_analys_gemm(p, g, gs, q, qs, nf, s)) return;
+  if (ts_launch_leg_analys_gemm(p, g, gs, q, qs, nf, s)) return ts_tc_size_wimg(p, nf, s);
   if (p->precision != TS_PREC_FP32) return ts_launch_leg_analys_tc(p, g, gs, q, qs, nf, s);
   int K, W;
   pick_kw(p->nh, K, W);

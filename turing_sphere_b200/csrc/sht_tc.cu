@@ -576,6 +576,16 @@ size_t ts_tc_wimg_bytes(ts_plan p, int nfields, int fpb) {
   return (size_t)(p->mmax + 1) * nfb * 2 * ts_tc_tab(p).nLC * 16384;
 }
 
+void ts_tc_size_qimg(ts_plan p, int nf, cudaStream_t s) {
+  if (!p->tc || ts_capturing(s)) return;
+  ensure_zeroed(static_cast<ts_tc_tables *>(p->tc)->qimg, ts_tc_qimg_bytes(p, nf), s);
+}
+
+void ts_tc_size_wimg(ts_plan p, int nf, cudaStream_t s) {
+  if (!p->tc || ts_capturing(s)) return;
+  ensure_zeroed(static_cast<ts_tc_tables *>(p->tc)->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
+}
+
 void ts_launch_qimage(ts_plan p, const TsFields &q, int nf, char *img, cudaStream_t s) {
   const int nfb = (nf + TS_TC_FIELDS - 1) / TS_TC_FIELDS;
   dim3 grid(ts_tc_tab(p).nchunks, nfb);
@@ -673,9 +683,12 @@ void ts_launch_leg_analys_tc(ts_plan p, const float2 *g, long gs, float2 *out, l
 // allows it, else spat -> G scratch -> w image; then -> q
 void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf, cudaStream_t s) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
-  if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s)) {
+  const size_t gbytes = sizeof(float2) * (size_t)(p->mmax + 1) * p->nlat * nf;
+  // (under capture only with the scratch there; the contraction needs none)
+  if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s) && (gbytes <= t->gscratch.cap || !ts_capturing(s))) {
     const long field = (long)(p->mmax + 1) * p->nlat;
-    t->gscratch.ensure(sizeof(float2) * field * nf);
+    ts_tc_size_wimg(p, nf, s);
+    t->gscratch.ensure(gbytes);
     ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
     ts_launch_leg_analys_gemm(p, (const float2 *)t->gscratch.p, field, (float2 *)qlm, p->nlm, nf, s);
     return;
@@ -683,7 +696,7 @@ void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf
   ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
   if (!ts_launch_fourier_analys_w(p, spat, ss, nf, TS_TC_FIELDS, (char *)t->wimg.p, s)) {
     const long field = (long)(p->mmax + 1) * p->nlat;
-    t->gscratch.ensure(sizeof(float2) * field * nf);
+    t->gscratch.ensure(gbytes);
     ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
     ts_launch_wimage(p, (const float2 *)t->gscratch.p, field, nf, TS_TC_FIELDS, (char *)t->wimg.p, s);
   }
