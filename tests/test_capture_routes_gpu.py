@@ -63,3 +63,33 @@ def test_capture_after_a_smaller_batch(device, parity, call, warm, batch):
     for f in (0, batch - 1):
         parity(f"captured {call} of {batch} after {warm}: field {f}", O.rel_l2(got[f].cpu().numpy(), want), 1e-5)
     plan.destroy()
+
+
+def test_captured_analysis_outlives_a_larger_call(device, parity):
+    """A captured analysis of 4 fields replays after a call of 16 and one of
+    64 on the same plan: the scratch it holds does not move for them."""
+    import torch
+    plan = ShtPlan.create(device, ShtConfig(LMAX, LMAX, NLAT, NPHI), {"precision": "tf32x3"})
+    ref = O.ShtReference(LMAX, LMAX, NLAT, NPHI)
+    q = spectrum(LMAX, LMAX, 5)
+    grid = ref.synth(q.astype(np.float64)).astype(np.float32)
+    spat = torch.from_numpy(np.tile(grid, (64, 1))).cuda()
+    out = torch.zeros(64, q.size, device="cuda")
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    plan.analys_dev(spat.data_ptr(), out.data_ptr(), 4, stream.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        plan.analys_dev(spat.data_ptr(), out.data_ptr(), 4, stream.cuda_stream)
+    free = torch.cuda.mem_get_info()[0]
+    for batch in (16, 64):
+        plan.analys_dev(spat.data_ptr(), out.data_ptr(), batch, stream.cuda_stream)
+        torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free  # nothing was allocated or moved
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    want = ref.analys(grid.astype(np.float64))
+    for f in (0, 3):
+        parity(f"captured analys of 4 after 16 and 64: field {f}", O.rel_l2(out[f].cpu().numpy(), want), 1e-5)
+    plan.destroy()

@@ -132,6 +132,8 @@ bool lg_few_analys(ts_plan p, int nf) {
 // a Brusselator's steady state), so the contraction's 1e-6 is up to 4e-4 of it
 // (lmax 235) and the gradient of an instance would change by as much with the
 // number of instances beside it.
+int ts_lg_most_analys(ts_plan p) { return lg_bytes(p) < (size_t)2 << 20 ? 48 : 16; }
+
 bool ts_lg_use(ts_plan p, int nf, bool analysis) {
   const size_t bytes = lg_bytes(p);
   if (!lg_fits(p)) return false;
@@ -139,7 +141,7 @@ bool ts_lg_use(ts_plan p, int nf, bool analysis) {
     // the adjoint of a model takes the contraction whatever the batch; the test
     // hook is about the tensor-core kernels
     if (p->in_adjoint || ts_tc_stalled(p)) return false;
-    if (analysis) return nf <= (bytes < (size_t)2 << 20 ? 48 : 16);
+    if (analysis) return nf <= ts_lg_most_analys(p);
     return nf <= (bytes <= (size_t)64 << 20 ? 48 : bytes <= (size_t)256 << 20 ? 32 : 16);
   }
   if (bytes < (size_t)384 << 10) return nf >= 8;

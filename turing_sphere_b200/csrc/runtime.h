@@ -200,6 +200,7 @@ void ts_launch_leg_synth_plain(ts_plan p, const TsFields &q, float2 *fm, long fm
 void ts_lg_init(ts_plan p, cudaStream_t s);
 bool ts_lg_prepare(ts_plan p, cudaStream_t s);  // the table is there (made now if it can be)
 bool ts_lg_use(ts_plan p, int nf, bool analysis);
+int ts_lg_most_analys(ts_plan p);  // fields of a tensor-core plan's analysis that take them
 bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fm_stride,
                               int nfields, cudaStream_t s);
 bool ts_launch_leg_analys_gemm(ts_plan p, const float2 *g, long g_stride, float2 *q, long q_stride,

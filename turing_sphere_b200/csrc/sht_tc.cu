@@ -683,12 +683,14 @@ void ts_launch_leg_analys_tc(ts_plan p, const float2 *g, long gs, float2 *out, l
 // allows it, else spat -> G scratch -> w image; then -> q
 void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf, cudaStream_t s) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
-  const size_t gbytes = sizeof(float2) * (size_t)(p->mmax + 1) * p->nlat * nf;
+  const size_t gfield = sizeof(float2) * (size_t)(p->mmax + 1) * p->nlat, gbytes = gfield * nf;
   // (under capture only with the scratch there; the contraction needs none)
   if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s) && (gbytes <= t->gscratch.cap || !ts_capturing(s))) {
     const long field = (long)(p->mmax + 1) * p->nlat;
     ts_tc_size_wimg(p, nf, s);
-    t->gscratch.ensure(gbytes);
+    // for the most fields that come here at once: a captured call's scratch must
+    // not move when a larger call follows, as the image does not within 64 fields
+    t->gscratch.ensure(gfield * ts_lg_most_analys(p));
     ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
     ts_launch_leg_analys_gemm(p, (const float2 *)t->gscratch.p, field, (float2 *)qlm, p->nlm, nf, s);
     return;
