@@ -1,0 +1,43 @@
+"""A tensor-core plan that has no memory for the FP32 products' tables when a
+small batch first wants them stays with the contraction: the call succeeds
+and no later one tries the allocation again."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from turing_sphere_b200 import ShtConfig, ShtPlan
+
+from .test_leg_gemm_gpu import spectrum
+
+pytestmark = pytest.mark.gpu
+
+
+def test_no_memory_for_the_tables(device, parity):
+    import torch
+    lmax, nlat, nphi = 511, 768, 1536  # 415 MB of tables
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": "tf32x3"})
+    q = spectrum(lmax, lmax, 1)
+    src = torch.from_numpy(np.tile(q, (64, 1))).cuda()
+    grid = torch.empty(64, nlat * nphi, device="cuda")
+    torch.cuda.synchronize()
+    plan.synth_dev(src.data_ptr(), grid.data_ptr(), 64)  # the contraction: its image and the scratch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (256 << 20), dtype=torch.uint8, device="cuda")
+    grid.zero_()
+    torch.cuda.synchronize()
+    plan.synth_dev(src.data_ptr(), grid.data_ptr(), 4)
+    device.sync()
+    first = grid[:4].clone()
+    parity("tf32x3 lmax511 B4 synth without tables", O.rel_l2(
+        first[3].cpu().numpy(), O.ShtReference(lmax, lmax, nlat, nphi).synth(q.astype(np.float64))), 1e-5)
+    del ballast
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    grid.zero_()
+    torch.cuda.synchronize()
+    plan.synth_dev(src.data_ptr(), grid.data_ptr(), 4)
+    device.sync()
+    assert torch.cuda.mem_get_info()[0] == free
+    assert torch.equal(grid[:4], first)
+    plan.destroy()

@@ -110,8 +110,8 @@ bool lg_few_analys(ts_plan p, int nf) {
 //              256: 742 | 181;  lmax 511: 1: 107 | 65, 8: 162 | 72
 // so all but a few fields on the smallest grids (a table under 384 KB), and
 // one or two fields' synthesis where the table comes from HBM (over 64 MB).
-// Above 512 MB the table is not made, nor above lmax 2047 (the recurrence
-// coefficients of an order are held in shared memory).
+// Above 512 MB a direction the tables are not made, nor above lmax 2047 (the
+// recurrence coefficients of an order are held in shared memory).
 //
 // On tensor-core plans the contraction works in blocks of 64 fields, so a small
 // batch is mostly padding there; the products read half the table bytes and
@@ -125,7 +125,9 @@ bool lg_few_analys(ts_plan p, int nf) {
 //              24: 966 | 1195
 // so the line lies at 16 fields, or for the synthesis at 48 where the table
 // stays in the L2 and 32 up to 256 MB, and for the smallest analyses at 48.
-// No table above 2 GB or lmax 1535.
+// No tables above 2 GB a direction or lmax 1535.  The two directions' are made
+// together by the first call that wants either (3.3 GB at lmax 1023 x 1536),
+// and a plan that has no memory for them then stays with the contraction.
 //
 // Not in a model's adjoint: a parameter's gradient can be a difference of large
 // terms (the derivative to dt sums the rate of change, A - (B + 1) u + u u v at
@@ -136,7 +138,7 @@ int ts_lg_most_analys(ts_plan p) { return lg_bytes(p) < (size_t)2 << 20 ? 48 : 1
 
 bool ts_lg_use(ts_plan p, int nf, bool analysis) {
   const size_t bytes = lg_bytes(p);
-  if (!lg_fits(p)) return false;
+  if (p->lg_none || !lg_fits(p)) return false;
   if (p->precision != TS_PREC_FP32) {
     // the adjoint of a model takes the contraction whatever the batch; the test
     // hook is about the tensor-core kernels
@@ -152,30 +154,37 @@ void ts_lg_init(ts_plan p, cudaStream_t s) {
   if (!lg_fits(p)) return;
   const size_t n = lg_floats(p), no = (size_t)(p->mmax + 1) * lg_nhp(p);
   float *tab = nullptr;
-  if (cudaMalloc(&tab, 2 * sizeof(float) * n + sizeof(int) * no) != cudaSuccess) {
+  const cudaError_t e = cudaMalloc(&tab, 2 * sizeof(float) * n + sizeof(int) * no);
+  if (e != cudaSuccess) {
     (void)cudaGetLastError();
+    p->lg_none = e == cudaErrorMemoryAllocation;
     return;
   }
-  p->lg_tab = tab;
   int *onset = (int *)(tab + 2 * n);
   const int nhp = lg_nhp(p), pairs = 2 * lg_k16(p->lmax, 0, 0) + 4;
+  const dim3 grid(nhp / 64, p->mmax + 1);
+  try {
+    if (p->precision == TS_PREC_FP32) {
+      const size_t smem = sizeof(float2) * pairs;
+      ts_leg_ptab_f32<false><<<grid, 64, smem, s>>>(p->leg, nhp, tab, onset);
+      TS_CUDA(cudaGetLastError());
+      ts_leg_ptab_f32<true><<<grid, 64, smem, s>>>(p->leg, nhp, tab + n, onset);
+    } else {
+      const size_t smem = sizeof(double2) * pairs;
+      ts_leg_ptab_f64<false><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
+                                                    tab, onset);
+      TS_CUDA(cudaGetLastError());
+      ts_leg_ptab_f64<true><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
+                                                   tab + n, onset);
+    }
+    TS_CUDA(cudaGetLastError());
+  } catch (...) {  // a table that is not written is no table
+    cudaFree(tab);
+    throw;
+  }
+  p->lg_tab = tab;
   p->lg_syn = TsLegGemmTab{tab, onset, nhp};
   p->lg_ana = TsLegGemmTab{tab + n, onset, nhp};
-  const dim3 grid(nhp / 64, p->mmax + 1);
-  if (p->precision == TS_PREC_FP32) {
-    const size_t smem = sizeof(float2) * pairs;
-    ts_leg_ptab_f32<false><<<grid, 64, smem, s>>>(p->leg, nhp, tab, onset);
-    TS_CUDA(cudaGetLastError());
-    ts_leg_ptab_f32<true><<<grid, 64, smem, s>>>(p->leg, nhp, tab + n, onset);
-  } else {
-    const size_t smem = sizeof(double2) * pairs;
-    ts_leg_ptab_f64<false><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
-                                                  tab, onset);
-    TS_CUDA(cudaGetLastError());
-    ts_leg_ptab_f64<true><<<grid, 64, smem, s>>>(p->d_x64, p->d_ab64, p->d_amm64, p->lmax, p->nh, nhp,
-                                                 tab + n, onset);
-  }
-  TS_CUDA(cudaGetLastError());
 }
 
 bool ts_launch_leg_synth_gemm(ts_plan p, const TsFields &q, float2 *fm, long fs, int nf,

@@ -147,6 +147,7 @@ struct ts_plan_s {
   // FP32 Legendre products (leg_gemm.cu): the tables of Legendre values of the
   // two directions (null: not made, or they do not fit)
   float *lg_tab = nullptr;
+  bool lg_none = false;  // there was no memory for them: not asked for again
   TsLegGemmTab lg_syn{}, lg_ana{};
   // tensor-core tables (precision != FP32)
   void *tc = nullptr;
