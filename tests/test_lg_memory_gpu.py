@@ -41,3 +41,30 @@ def test_no_memory_for_the_tables(device, parity):
     assert torch.cuda.mem_get_info()[0] == free
     assert torch.equal(grid[:4], first)
     plan.destroy()
+
+
+def test_no_memory_for_the_scratch(device, parity):
+    """With the tables made and the operand image in place, a small analysis
+    that finds no memory for the products' scratch (50 MB) runs as the
+    contraction."""
+    import torch
+    lmax, nlat, nphi = 511, 768, 1536
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi), {"precision": "tf32x3"})
+    ref = O.ShtReference(lmax, lmax, nlat, nphi)
+    q = spectrum(lmax, lmax, 2)
+    grid = ref.synth(q.astype(np.float64)).astype(np.float32)
+    spat = torch.from_numpy(np.tile(grid, (64, 1))).cuda()
+    spec = torch.from_numpy(np.tile(q, (64, 1))).cuda()
+    fm = torch.empty(4, (lmax + 1) * nlat * 2, device="cuda")
+    torch.cuda.synchronize()
+    plan.stage_dev("legSynth", spec.data_ptr(), fm.data_ptr(), 4)    # the tables
+    plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 64)            # the image
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+    plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 4)
+    device.sync()
+    del ballast
+    parity("tf32x3 lmax511 B4 analys without scratch",
+           O.rel_l2(spec[3].cpu().numpy(), ref.analys(grid.astype(np.float64))), 1e-5)
+    plan.destroy()

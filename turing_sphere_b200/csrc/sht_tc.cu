@@ -683,14 +683,26 @@ void ts_launch_leg_analys_tc(ts_plan p, const float2 *g, long gs, float2 *out, l
 // allows it, else spat -> G scratch -> w image; then -> q
 void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf, cudaStream_t s) {
   auto *t = static_cast<ts_tc_tables *>(p->tc);
-  const size_t gfield = sizeof(float2) * (size_t)(p->mmax + 1) * p->nlat, gbytes = gfield * nf;
-  // (under capture only with the scratch there; the contraction needs none)
-  if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s) && (gbytes <= t->gscratch.cap || !ts_capturing(s))) {
+  const size_t gfield = sizeof(float2) * (size_t)(p->mmax + 1) * p->nlat;
+  // The products' scratch is made for the most fields that they take at once: a
+  // captured call's scratch must not move when a larger call follows, as the
+  // image does not within 64 fields.  Where it cannot be had (under capture, or
+  // memory is short) the contraction, which needs none, takes the call.
+  auto scratch = [&] {
+    const size_t bytes = gfield * ts_lg_most_analys(p);
+    if (bytes <= t->gscratch.cap) return true;
+    if (ts_capturing(s)) return false;
+    try {
+      t->gscratch.ensure(bytes);
+    } catch (const ts_exc &) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    return true;
+  };
+  if (ts_lg_use(p, nf, true) && ts_lg_prepare(p, s) && scratch()) {
     const long field = (long)(p->mmax + 1) * p->nlat;
     ts_tc_size_wimg(p, nf, s);
-    // for the most fields that come here at once: a captured call's scratch must
-    // not move when a larger call follows, as the image does not within 64 fields
-    t->gscratch.ensure(gfield * ts_lg_most_analys(p));
     ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
     ts_launch_leg_analys_gemm(p, (const float2 *)t->gscratch.p, field, (float2 *)qlm, p->nlm, nf, s);
     return;
@@ -698,7 +710,7 @@ void ts_analys_tc_full(ts_plan p, const float *spat, long ss, float *qlm, int nf
   ensure_zeroed(t->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
   if (!ts_launch_fourier_analys_w(p, spat, ss, nf, TS_TC_FIELDS, (char *)t->wimg.p, s)) {
     const long field = (long)(p->mmax + 1) * p->nlat;
-    t->gscratch.ensure(gbytes);
+    t->gscratch.ensure(gfield * nf);
     ts_launch_fourier_analys(p, spat, ss, (float2 *)t->gscratch.p, field, nf, s);
     ts_launch_wimage(p, (const float2 *)t->gscratch.p, field, nf, TS_TC_FIELDS, (char *)t->wimg.p, s);
   }
