@@ -1853,6 +1853,27 @@ int ts_model_group_destroy(ts_group g) {
   return TS_OK;
 }
 
+namespace {
+// at the end of a call, also of one that fails, small workspaces stay for the
+// next one and large ones go back
+struct AdjMemory {
+  Adjoint &A;
+  explicit AdjMemory(Adjoint &a) : A(a) {}
+  ~AdjMemory() {
+    const size_t keep = (size_t)256 << 20;
+    if (A.ck.cap + A.seg.cap > keep) {
+      A.ck.release();
+      A.seg.release();
+    }
+    if (A.lam.cap + A.cur.cap > keep) {
+      adj_drop_graphs(A);
+      A.lam.release();
+      A.cur.release();
+    }
+  }
+};
+}  // namespace
+
 int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *final_bar,
                               float *init_bar, double *param_bar) {
   TSM_BEGIN(m)
@@ -1864,6 +1885,7 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   const int B = m->batch, ns = (int)m->state.size();
   const long sz = 2 * m->plan->nlm * (long)B;  // floats of one state, all instances
   const int nseg = (nsteps + every - 1) / every;
+  const AdjMemory memory(A);
   // checkpoints [segment][state], segment states [step][state], cotangents
   // [state], and the states [state] a tape starts from
   A.ck.ensure(sizeof(float) * sz * ns * nseg);
@@ -1933,16 +1955,6 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
                             cudaMemcpyDeviceToHost, st));
   TS_CUDA(cudaStreamSynchronize(st));
   TS_CUDA(cudaGetLastError());
-  // small workspaces stay for the next call, large ones go back
-  if (A.ck.cap + A.seg.cap > (size_t)256 << 20) {
-    A.ck.release();
-    A.seg.release();
-  }
-  if (A.lam.cap + A.cur.cap > (size_t)256 << 20) {
-    adj_drop_graphs(A);
-    A.lam.release();
-    A.cur.release();
-  }
   TSM_END
 }
 
