@@ -624,13 +624,19 @@ constexpr long ts_f2_smem_bytes(int nb) {
 // fields at lmax 511 (nphi 1536): synthesis 178 us with 16 rows, 159 with 8 and
 // two CTAs, 141 with three.  The fused phase keeps every species' P grid points
 // of a row in registers: with one or two species, CTAs of at most 256 threads
-// are held to 128 registers (they would take 142), so that two share an SM;
-// larger CTAs and more species get what they need (168 at P = 24, where two
-// CTAs would spill).  The phase of 256 Brusselator instances at lmax 127
-// (P = 16): one CTA an SM 150 us, two 110 us.
+// are held to what lets two share an SM where its shared memory holds two
+// (P = 16 to 128 registers, they would take 142; P = 24 on 8 rows to 168 of
+// 206; P = 32 on 8 rows to 128 of 255, with 150 bytes of spills); larger CTAs
+// and more species get what they need.  One CTA an SM | two: the phase of 256
+// Brusselator instances at lmax 127 (P = 16) 150 us | 110; whole steps of
+// nphi 1536 x 2 (P = 32, 8 rows) 76 | 69, nphi 1024 x 4 45 | 40; nphi 2048
+// (Q = 32: one CTA fits, so only the spills would be left) x 64 2181 | 2479.
 #define TS_F2_MINB(P, Q, R) \
   ((P) <= 24 ? 1152 / ((P) * (R)) : (P) == 32 && (R) == 8 ? ((Q) <= 24 ? 3 : 2) : 1)
-#define TS_F2_PHASE_MINB(NB, P, R) ((NB) <= 2 && (P) * (R) <= 256 ? 2 : 1)
+template <class C>
+constexpr int ts_f2_phase_minb(int nb) {
+  return nb <= 2 && C::P * C::R <= 256 && 2 * (ts_f2_smem_bytes<C>(nb) + 1024) <= 228 * 1024 ? 2 : 1;
+}
 
 // fm[field][m][lat] -> spat[field][lat][phi].  grid = (ceil(nlat/R), fields),
 // block = P*R.  Rows leave by bulk copies when the field's grid is 16-byte
@@ -845,7 +851,7 @@ TS_DEV void ts_f2_groups(F &&f) {
 // pair of barriers and one batch of loads per pair (the registers of two
 // P-point rows per thread are what the middle section holds anyway).
 template <class Prog, int P, int Q, int R, bool PAIRED>
-__global__ void __launch_bounds__(P *R, TS_F2_PHASE_MINB(Prog::NSYN > Prog::NANA ? Prog::NSYN : Prog::NANA, P, R))
+__global__ void __launch_bounds__(P *R, ts_f2_phase_minb<TsF2<P, Q, R>>(Prog::NSYN > Prog::NANA ? Prog::NSYN : Prog::NANA))
 ts_f2_phase(TsFftTab ft, TsPhaseIO io) {
   using C = TsF2<P, Q, R>;
   constexpr int NSYN = Prog::NSYN, NGIN = Prog::NGIN, NANA = Prog::NANA, NGOUT = Prog::NGOUT;
