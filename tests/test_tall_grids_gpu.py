@@ -72,3 +72,23 @@ def test_one_instance_beyond_the_shared_memory(device, parity):
         parity(f"fp32 schnakenberg lmax31 nlat13600 {name}", O.rel_l2(gpu.read(name), want[i]), 1e-4)
     gpu.destroy()
     plan.destroy()
+
+
+@pytest.mark.parametrize("lmax,nlat", [(3, 641), (3, 670), (3, 770), (3, 1566), (1, 3074), (1, 3134)])
+def test_recurrence_analysis_between_its_shapes(device, parity, lmax, nlat):
+    """Northern latitudes between the recurrence kernel's shapes (grids small
+    enough in lmax to take it): one and three fields against the oracle."""
+    import torch
+    nphi = 32
+    plan = ShtPlan.create(device, ShtConfig(lmax, lmax, nlat, nphi))
+    ref = O.ShtReference(lmax, lmax, nlat, nphi)
+    for batch in (1, 3):
+        grid = np.random.default_rng(nlat).standard_normal((batch, nlat * nphi)).astype(np.float32)
+        src, out = torch.from_numpy(grid).cuda(), torch.empty(batch, 2 * plan.nlm, device="cuda")
+        torch.cuda.synchronize()
+        plan.analys_dev(src.data_ptr(), out.data_ptr(), batch)
+        device.sync()
+        for f in range(batch):
+            want = ref.analys(grid[f].astype(np.float64))
+            parity(f"fp32 lmax{lmax} nlat{nlat} B{batch} analys {f}", O.rel_l2(out[f].cpu().numpy(), want), 1e-5)
+    plan.destroy()

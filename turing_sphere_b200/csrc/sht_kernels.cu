@@ -270,6 +270,10 @@ void pick_kw(int nh, int &K, int &W) {
   if (best == (1 << 30)) {  // tiny grids: one warp, one latitude per lane
     K = 1;
     W = (nh + 31) / 32;
+    if (W > 8) {  // more than 256: no shape under 1/8 idle, and a CTA has up to 8 warps
+      K = 8;
+      W = (nh + 255) / 256;
+    }
   }
 }
 
