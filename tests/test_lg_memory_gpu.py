@@ -65,6 +65,7 @@ def test_no_memory_for_the_scratch(device, parity):
     plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 4)
     device.sync()
     del ballast
+    torch.cuda.empty_cache()
     parity("tf32x3 lmax511 B4 analys without scratch",
            O.rel_l2(spec[3].cpu().numpy(), ref.analys(grid.astype(np.float64))), 1e-5)
     plan.destroy()

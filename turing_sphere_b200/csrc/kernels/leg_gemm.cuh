@@ -454,12 +454,13 @@ ts_leg_synth_gemm(TsLegTab t, TsLegGemmTab g, TsFields q, float2 *__restrict__ f
 // ---------------------------------------------------------------- analysis
 //
 // grid = (ceil((lmax + 1) / 128), ceil(nfields / per_cta), mmax + 1), per_cta
-// <= NF whole instances of Epi::NA fields: the degrees of an order are split evenly over its ceil(K / 128) CTAs; the others leave
-// at once.  A CTA's degrees of a parity (a multiple of 8 up to 32, of 16 up to
-// 64) are one or two equal blocks of 8 NP; with two blocks of each parity a
-// warp takes one, with one block two warps share it: each takes half of every
-// stage's k-steps, and the halves are added up at the end.  Latitudes before
-// the first value of a warp's degrees are left out.
+// <= NF whole instances of Epi::NA fields: the degrees of an order are split
+// evenly over its ceil(K / 128) CTAs; the others leave at once.  A CTA's degrees
+// of a parity (a multiple of 8 up to 32, of 16 up to 64) are one or two equal
+// blocks of 8 NP; with two blocks of each parity a warp takes one, with one
+// block two warps share it: each takes half of every stage's k-steps, and the
+// halves are added up at the end.  Latitudes before the first value of a warp's
+// degrees are left out.
 template <int NCOL, class Epi>
 __global__ void __launch_bounds__(TS_LG_THREADS, 4)
 ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *gm, long g_stride, Epi epi,
@@ -648,10 +649,11 @@ ts_leg_analys_gemm(TsLegTab t, TsLegGemmTab g, const float2 *gm, long g_stride, 
 //
 // One or two fields: every table value meets two or four numbers, so the
 // products are bound by reading the table (25 MB a direction at lmax 255, from
-// the L2) and by the latency of a CTA's few stages.  No staging then: a warp's lanes read whole rows of the table
-// straight into registers, pairs of neighbours each, with eight rows in flight,
-// and the columns come as broadcasts from shared memory.  The rows of a CTA are
-// dealt out to its warps, whose sums are added up at the end.
+// the L2) and by the latency of a CTA's few stages.  No staging then: a warp's
+// lanes read whole rows of the table straight into registers, pairs of
+// neighbours each, with eight rows in flight, and the columns come as broadcasts
+// from shared memory.  The rows of a CTA are dealt out to its warps, whose sums
+// are added up at the end.
 
 // a load of what the kernel before this one wrote: not through the read-only
 // path, and not moved ahead of ts_grid_wait()

@@ -577,13 +577,17 @@ size_t ts_tc_wimg_bytes(ts_plan p, int nfields, int fpb) {
 }
 
 void ts_tc_size_qimg(ts_plan p, int nf, cudaStream_t s) {
-  if (!p->tc || ts_capturing(s)) return;
-  ensure_zeroed(static_cast<ts_tc_tables *>(p->tc)->qimg, ts_tc_qimg_bytes(p, nf), s);
+  if (!p->tc) return;
+  ts_dbuf &b = static_cast<ts_tc_tables *>(p->tc)->qimg;
+  const size_t bytes = ts_tc_qimg_bytes(p, nf);
+  if (bytes > b.cap && !ts_capturing(s)) ensure_zeroed(b, bytes, s);
 }
 
 void ts_tc_size_wimg(ts_plan p, int nf, cudaStream_t s) {
-  if (!p->tc || ts_capturing(s)) return;
-  ensure_zeroed(static_cast<ts_tc_tables *>(p->tc)->wimg, ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS), s);
+  if (!p->tc) return;
+  ts_dbuf &b = static_cast<ts_tc_tables *>(p->tc)->wimg;
+  const size_t bytes = ts_tc_wimg_bytes(p, nf, TS_TC_FIELDS);
+  if (bytes > b.cap && !ts_capturing(s)) ensure_zeroed(b, bytes, s);
 }
 
 void ts_launch_qimage(ts_plan p, const TsFields &q, int nf, char *img, cudaStream_t s) {
