@@ -1,6 +1,8 @@
 """A tensor-core plan that has no memory for the FP32 products' tables when a
 small batch first wants them stays with the contraction: the call succeeds
 and no later one tries the allocation again."""
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -12,6 +14,20 @@ from .test_leg_gemm_gpu import spectrum
 pytestmark = pytest.mark.gpu
 
 
+@contextlib.contextmanager
+def little_memory(left):
+    """All but `left` bytes of the GPU's free memory taken for the block."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ballast = [torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")]
+    try:
+        yield
+    finally:
+        ballast.clear()
+        torch.cuda.empty_cache()
+
+
 def test_no_memory_for_the_tables(device, parity):
     import torch
     lmax, nlat, nphi = 511, 768, 1536  # 415 MB of tables
@@ -21,18 +37,13 @@ def test_no_memory_for_the_tables(device, parity):
     grid = torch.empty(64, nlat * nphi, device="cuda")
     torch.cuda.synchronize()
     plan.synth_dev(src.data_ptr(), grid.data_ptr(), 64)  # the contraction: its image and the scratch
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (256 << 20), dtype=torch.uint8, device="cuda")
     grid.zero_()
-    torch.cuda.synchronize()
-    plan.synth_dev(src.data_ptr(), grid.data_ptr(), 4)
-    device.sync()
+    with little_memory(256 << 20):
+        plan.synth_dev(src.data_ptr(), grid.data_ptr(), 4)
+        device.sync()
     first = grid[:4].clone()
     parity("tf32x3 lmax511 B4 synth without tables", O.rel_l2(
         first[3].cpu().numpy(), O.ShtReference(lmax, lmax, nlat, nphi).synth(q.astype(np.float64))), 1e-5)
-    del ballast
-    torch.cuda.empty_cache()
     free = torch.cuda.mem_get_info()[0]
     grid.zero_()
     torch.cuda.synchronize()
@@ -59,13 +70,9 @@ def test_no_memory_for_the_scratch(device, parity):
     torch.cuda.synchronize()
     plan.stage_dev("legSynth", spec.data_ptr(), fm.data_ptr(), 4)    # the tables
     plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 64)            # the image
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
-    plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 4)
-    device.sync()
-    del ballast
-    torch.cuda.empty_cache()
+    with little_memory(24 << 20):
+        plan.analys_dev(spat.data_ptr(), spec.data_ptr(), 4)
+        device.sync()
     parity("tf32x3 lmax511 B4 analys without scratch",
            O.rel_l2(spec[3].cpu().numpy(), ref.analys(grid.astype(np.float64))), 1e-5)
     plan.destroy()
