@@ -57,8 +57,9 @@ enum ts_status {
 
 /* Plan flags (bitwise OR). */
 enum ts_plan_flags {
-  TS_PREC_FP32 = 0,        /* plain FP32 on-the-fly recurrence (default) */
-  TS_PREC_TF32X3 = 1,      /* tcgen05 tensor-core Legendre, 3-pass split TF32 */
+  TS_PREC_FP32 = 0,        /* plain FP32 recurrence, by way of a table where it fits (default) */
+  TS_PREC_TF32X3 = 1,      /* tcgen05 tensor-core Legendre, 3-pass split TF32 (small
+                              batches: FP32 products with the FP64 functions rounded once) */
   TS_PREC_BF16X3 = 2,      /* tcgen05 tensor-core Legendre, 3-pass split BF16 */
   TS_PREC_MASK = 0xF,
   TS_CHECK_SOURCE = 0x100, /* ts_model_check: return the generated source */
@@ -109,7 +110,9 @@ typedef struct ts_plan_info {
   int fourier;    /* TS_FOURIER_FFT or TS_FOURIER_DFT in use */
   int fft_stages; /* Stockham stages of the nphi/2-point FFT (0 for DFT) */
   int fft_radix[16];
-  long table_bytes; /* tensor-core P tables in device memory (0 for FP32) */
+  long table_bytes; /* tensor-core P tables in device memory (0 for FP32; the FP32
+                       products' tables of a plan, up to 1 GB, on a tensor-core
+                       plan from its first small batch on up to 4 GB, are beside it) */
   /* kernel shapes in use (chosen by TS_PLAN_AUTOTUNE, else the defaults) */
   int tc_lat_tile;   /* tensor-core synthesis: latitudes per tile (0 for FP32) */
   int tc_deg_tile;   /* tensor-core analysis: degrees per tile (0 for FP32) */
@@ -151,8 +154,8 @@ int ts_sht_analys_dev(ts_plan plan, const float *spat, float *qlm, int batch, vo
 /* Allocation-free synthesis.  No counterpart in the reference: it exists for
  * callers that cannot let the library call cudaMalloc (hosts that own every
  * device allocation, or loops that must not stall on cudaMalloc's implicit
- * device synchronisation).  Same inputs, outputs and result as
- * ts_sht_synth_dev, but the Fourier intermediate lives in a fixed 16 MiB
+ * device synchronisation).  Same inputs, outputs and (to FP32 rounding) result
+ * as ts_sht_synth_dev, but the Fourier intermediate lives in a fixed 16 MiB
  * array compiled into the library (held on every GPU that loads it until the
  * process exits), so the call allocates nothing.  A batch whose intermediate
  * exceeds 16 MiB ((mmax+1)*nlat*8 bytes per field) fails with TS_ERR_SIZE.
@@ -278,8 +281,9 @@ int ts_model_group_destroy(ts_group group);
 
 /* Forward/backward pair of the adjoint (no reference counterpart; the
  * autograd.Function of this path).  Advances the model nsteps steps from its
- * current state, as ts_model_step does, keeping a checkpoint of the state
- * every `every` steps; then runs the hand-written adjoint of the step (the
+ * current state, as ts_model_step does (on a tensor-core plan with the
+ * contraction for every batch, so that small batches end within its rounding
+ * of ts_model_step), keeping a checkpoint of the state every `every` steps; then runs the hand-written adjoint of the step (the
  * transposed transforms, the symbolically differentiated element-wise
  * statements and the implicit diffusion solve) backwards, replaying each
  * segment from its checkpoint.  final_bar: dL/d(final state), host
@@ -312,8 +316,8 @@ int ts_model_describe(ts_model model, int which, char *buf, size_t cap);
 int ts_model_source(ts_model model, char *buf, size_t cap);
 /* Element-wise statements (the reference's kernel count, the fusion guard of
  * test/modelChecks.ts:17-21) and CUDA kernel launches per call (on a
- * tensor-core plan a Legendre synthesis is two: the operand relayout and the
- * tcgen05 contraction). */
+ * tensor-core plan a large batch's Legendre synthesis is two: the operand
+ * relayout and the tcgen05 contraction). */
 int ts_model_counts(ts_model model, int which, int *kernels, int *launches);
 
 /* Everything ts_model_compile does short of the GPU — parse, specialise,

@@ -40,10 +40,7 @@ def test_both_graphs_run_on_a_fresh_model(device, precision, steps, every):
     assert (replayed, reverse) == (0, 0)
     got, replayed, reverse = fresh(True)
     segments = -(-steps // every)
-    replays = steps - segments
-    if precision == "tf32x3":  # the checkpoints' trajectory takes replayed steps too
-        replays += (segments - 1) * every
-    assert replayed == max(0, replays - 2)
+    assert replayed == max(0, steps - segments - 2)
     assert reverse == steps - 2
     for s in model.state:
         assert np.array_equal(got[0][s], want[0][s]), s

@@ -129,11 +129,13 @@ bool lg_few_analys(ts_plan p, int nf) {
 // together by the first call that wants either (3.3 GB at lmax 1023 x 1536),
 // and a plan that has no memory for them then stays with the contraction.
 //
-// Not in a model's adjoint: a parameter's gradient can be a difference of large
-// terms (the derivative to dt sums the rate of change, A - (B + 1) u + u u v at
-// a Brusselator's steady state), so the contraction's 1e-6 is up to 4e-4 of it
-// (lmax 235) and the gradient of an instance would change by as much with the
-// number of instances beside it.
+// Not in a model's forward_backward: a parameter's gradient can be a difference
+// of large terms (the derivative to dt sums the rate of change, A - (B + 1) u +
+// u u v at a Brusselator's steady state), so the contraction's 1e-6 is up to
+// 4e-4 of it (lmax 235), and the gradient of an instance would change by as much
+// with the number of instances beside it.  Even the rounding of a step's
+// statements, compiled otherwise, is 6e-5 (lmax 127): its forward steps are the
+// same kernels whatever the batch.
 int ts_lg_most_analys(ts_plan p) { return lg_bytes(p) < (size_t)2 << 20 ? 48 : 16; }
 
 bool ts_lg_use(ts_plan p, int nf, bool analysis) {

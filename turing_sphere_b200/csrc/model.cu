@@ -22,6 +22,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <optional>
 #include <set>
 #include <sstream>
 
@@ -222,6 +223,7 @@ struct ts_model_s {
     std::vector<float *> key;
     int nsteps;
     cudaGraphExec_t exec;
+    bool in_adjoint;  // captured for forward_backward (see ts_lg_use)
   };
   std::vector<StepGraph> graphs;
   bool use_graphs = true;
@@ -516,10 +518,14 @@ void schedule(ts_model m, Program &P, bool is_step) {
       int fP = 0, fQ = 0, fR = 0;
       const int nb = std::max<int>({(int)S.size(), (int)A.size(), 1});
       if (ts_f2_phase_shape(p, &fP, &fQ)) fR = ts_f2_phase_rows(p, nb, m->batch, &st.smem);
-      // the smallest tile of the products holds 8 fields, whole instances
-      lg = !A.empty() && A.size() <= 8 && ts_lg_use(p, m->batch * (int)A.size(), true) &&
+      // The products on FP32 plans only: a tensor-core plan's adjoint needs the
+      // contraction (see ts_lg_use), and one compiled step serves it and the
+      // steps, whose synthesis alone takes the products of a small batch.  The
+      // smallest tile of the products holds 8 fields, whole instances.
+      lg = p->precision == TS_PREC_FP32 && !A.empty() && A.size() <= 8 &&
+           ts_lg_use(p, m->batch * (int)A.size(), true) &&
            (m->host_only || ts_lg_prepare(p, m->ctx->stream));
-      const bool tcw = p->precision != TS_PREC_FP32 && !lg && fR && !A.empty();
+      const bool tcw = p->precision != TS_PREC_FP32 && fR && !A.empty();
       if (fR) {
         st.expr = "ts_f2_phase<" + pn + ", " + std::to_string(fP) + ", " + std::to_string(fQ) +
                   ", " + std::to_string(fR) + ", " + (tcw ? "true" : "false") + ">";
@@ -549,7 +555,7 @@ void schedule(ts_model m, Program &P, bool is_step) {
     // 64-field block for one coefficient; with many instances that loop of
     // dependent state loads is latency-bound, so the analysis only stores and
     // the spectral statements run as a coalesced element-wise stage (A).
-    const bool fuse_epi = p->precision == TS_PREC_FP32 || lg || m->batch * (long)A.size() <= 16;
+    const bool fuse_epi = p->precision == TS_PREC_FP32 || m->batch * (long)A.size() <= 16;
     for (size_t i = 0; i < f.body.size() && fuse_epi; i++) {
       const auto &s = f.body[i];
       if (done[i] || s.kind != tsm::Stmt::Elementwise || f.vars[s.out].dom != Dom::Spec) continue;
@@ -585,7 +591,7 @@ void schedule(ts_model m, Program &P, bool is_step) {
     st.wimg = P.stages.back().kind == Stage::Phase && P.stages.back().wimg;
     for (int v : sin) st.in.push_back(ref[v]);
     for (int v : sout) st.out.push_back(ref[v]);
-    const bool tc = p->precision != TS_PREC_FP32 && !lg;
+    const bool tc = p->precision != TS_PREC_FP32;
     if (tc) {
       st.per_cta = st.nana * (TS_TC_FIELDS / st.nana);  // whole instances per 64-field block
       if (st.per_cta == 0)
@@ -998,8 +1004,9 @@ void swap_states(ts_model m, int nsteps) {
 void run_steps_graphed(ts_model m, int nsteps) {
   cudaStream_t st = m->ctx->stream;
   const std::vector<float *> key = state_key(m);
+  const bool in_adjoint = m->plan->in_adjoint;
   for (auto &g : m->graphs)
-    if (g.nsteps == nsteps && g.key == key) {
+    if (g.nsteps == nsteps && g.key == key && g.in_adjoint == in_adjoint) {
       TS_CUDA(cudaGraphLaunch(g.exec, st));
       swap_states(m, nsteps);
       return;
@@ -1027,7 +1034,7 @@ void run_steps_graphed(ts_model m, int nsteps) {
     for (int i = 0; i < nsteps; i++) run_program(m, m->prog[1], st);
     return;
   }
-  m->graphs.push_back({key, nsteps, exec});
+  m->graphs.push_back({key, nsteps, exec, in_adjoint});
   TS_CUDA(cudaGraphLaunch(exec, st));
 }
 
@@ -1272,16 +1279,6 @@ struct AdjointScope {  // launches of this scope are the adjoint's
   explicit AdjointScope(ts_plan p_) : p(p_) { p->in_adjoint = true; }
   ~AdjointScope() { p->in_adjoint = false; }
 };
-
-// whether a step's transforms are, in part, the FP32 products of a small batch
-// on a tensor-core plan, and so not those of its adjoint
-bool step_takes_products(ts_model m) {
-  if (m->plan->precision == TS_PREC_FP32) return false;
-  for (auto &s : m->prog[1].stages)
-    if (s.lg.threads || (s.kind == Stage::LegSynth && ts_lg_use(m->plan, m->batch * s.nsyn, false)))
-      return true;
-  return false;
-}
 
 // the step's values from the states at `states[s]` ([instance][2 nlm] each)
 void adj_tape(ts_model m, const std::vector<const float *> &states, cudaStream_t st) {
@@ -1557,19 +1554,16 @@ int ts_model_compile(ts_plan plan, const char *source, const char *const *state,
       size_t wb = 0;
       for (auto &P : m->prog)
         for (auto &st : P.stages)
-          if (st.kind == Stage::LegAnalys && !st.lg.threads)
+          if (st.kind == Stage::LegAnalys)
             wb = std::max(wb, ts_tc_wimg_bytes(plan, batch * st.nana, st.per_cta));
       m->wimg.ensure(std::max<size_t>(wb, 16));
       TS_CUDA(cudaMemset(m->wimg.p, 0, m->wimg.cap));
-      bool image = false;  // some synthesis is the contraction
+      m->qimg.ensure(ts_tc_qimg_bytes(plan, batch * nsyn));
+      TS_CUDA(cudaMemset(m->qimg.p, 0, m->qimg.cap));
       for (auto &P : m->prog)
         for (auto &st : P.stages)
-          image = image || (st.kind == Stage::LegSynth &&
-                            !(ts_lg_use(plan, batch * st.nsyn, false) && ts_lg_prepare(plan, ctx->stream)));
-      if (image) {
-        m->qimg.ensure(ts_tc_qimg_bytes(plan, batch * nsyn));
-        TS_CUDA(cudaMemset(m->qimg.p, 0, m->qimg.cap));
-      }
+          if (st.kind == Stage::LegSynth && ts_lg_use(plan, batch * st.nsyn, false))
+            ts_lg_prepare(plan, ctx->stream);  // the products' tables, before the first step
     }
     m->stash.ensure(sizeof(float) * 2 * nlm * batch * nstate);
     m->h_prm.assign((size_t)std::max(nparams, 1) * batch, 0.0f);
@@ -1903,31 +1897,14 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
   auto copy = [&](float *dst, const float *src) {
     TS_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * sz * ns, cudaMemcpyDeviceToDevice, st));
   };
-  auto take_state = [&](float *dst) {  // the model's current states
-    for (int s = 0; s < ns; s++)
-      TS_CUDA(cudaMemcpyAsync(dst + (long)s * sz, m->host.at(m->state[s]).cur, sizeof(float) * sz,
-                              cudaMemcpyDeviceToDevice, st));
-  };
-  auto replay_step = [&] {  // the states in `cur` one step on
-    adj_graphed(m, A.fwd, st, [&] {
-      adj_tape(m, cur, st);
-      for (int s = 0; s < ns; s++)
-        TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
-                                cudaMemcpyDeviceToDevice, st));
-    });
-  };
-  if (nseg > 1 && step_takes_products(m)) {
-    // the checkpoints lie on the adjoint's own trajectory, which the step's
-    // products would leave by their difference to the contraction
-    take_state(pcur);
-    for (int g = 0; g < nseg; g++) {
-      copy(pck + (long)g * ns * sz, pcur);
-      for (int j = 0; j < every && g + 1 < nseg; j++) replay_step();
-    }
-    advance(m, nsteps);
-  } else {
+  {
+    // the checkpoints lie on the contraction's trajectory, as the tapes do
+    std::optional<AdjointScope> scope;
+    if (m->plan->precision != TS_PREC_FP32) scope.emplace(m->plan);
     for (int i = 0; i < nsteps; i += every) {
-      take_state(pck + (long)(i / every) * ns * sz);
+      for (int s = 0; s < ns; s++)
+        TS_CUDA(cudaMemcpyAsync(pck + ((long)(i / every) * ns + s) * sz, m->host.at(m->state[s]).cur,
+                                sizeof(float) * sz, cudaMemcpyDeviceToDevice, st));
       advance(m, std::min(every, nsteps - i));
     }
   }
@@ -1938,7 +1915,12 @@ int ts_model_forward_backward(ts_model m, int nsteps, int every, const float *fi
     copy(pcur, pck + (long)g * ns * sz);
     copy(pseg, pcur);
     for (int j = 1; j < len; j++) {  // replay the segment: the state before every step
-      replay_step();
+      adj_graphed(m, A.fwd, st, [&] {
+        adj_tape(m, cur, st);
+        for (int s = 0; s < ns; s++)
+          TS_CUDA(cudaMemcpyAsync(pcur + (long)s * sz, A.val[A.state_out[s]], sizeof(float) * sz,
+                                  cudaMemcpyDeviceToDevice, st));
+      });
       copy(pseg + (long)j * ns * sz, pcur);
     }
     for (int j = len - 1; j >= 0; j--) {
