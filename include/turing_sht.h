@@ -283,10 +283,10 @@ int ts_model_group_destroy(ts_group group);
  * autograd.Function of this path).  Advances the model nsteps steps from its
  * current state, as ts_model_step does (on a tensor-core plan with the
  * contraction for every batch, so that small batches end within its rounding
- * of ts_model_step), keeping a checkpoint of the state every `every` steps; then runs the hand-written adjoint of the step (the
- * transposed transforms, the symbolically differentiated element-wise
- * statements and the implicit diffusion solve) backwards, replaying each
- * segment from its checkpoint.  final_bar: dL/d(final state), host
+ * of ts_model_step), keeping a checkpoint of the state every `every` steps;
+ * then runs the hand-written adjoint of the step (the transposed transforms,
+ * the symbolically differentiated element-wise statements and the implicit
+ * diffusion solve) backwards, replaying each segment from its checkpoint.  final_bar: dL/d(final state), host
  * [state][instance][2 nlm] in the model's state order; init_bar receives
  * dL/d(initial state) in the same layout; param_bar (may be NULL) receives
  * dL/d(parameters), host double [instance][nparams]. */
