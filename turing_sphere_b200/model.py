@@ -208,8 +208,11 @@ class GpuModel:
             self.handle = None
 
     def __del__(self):
+        # the garbage collector may finalize the device of the same cycle (a
+        # script's globals at exit) before its models: their handles are dead then
         try:
-            self.destroy()
+            if self.device.handle:
+                self.destroy()
         except Exception:
             pass
 

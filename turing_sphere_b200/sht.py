@@ -212,7 +212,8 @@ class ShtPlan:
 
     def __del__(self):
         try:
-            self.destroy()
+            if self.device.handle:  # (see GpuModel.__del__)
+                self.destroy()
         except Exception:
             pass
 
